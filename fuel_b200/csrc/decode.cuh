@@ -34,6 +34,7 @@ struct DecodeParams {
   int64_t total_bytes;
   int k;
   int m;
+  int early_w;       // weights are streamed before the wait for the preceding kernel
   int row_bytes;
   int units_per_row;
   int rows_per_stage;
@@ -409,7 +410,8 @@ __global__ void __launch_bounds__(kDecodeThreads, 2) decode_matvec_kernel(const 
   pdl_launch_dependents();
 
   if (warp == kDecodeConsumerWarps) {
-    // ---------------- producer: weights never depend on the previous kernel, so no pdl_wait here
+    // ---------------- producer (with early_w the weights do not depend on the previous kernel)
+    if (!p.early_w) pdl_wait();
     if (lane == 0) {
       const int64_t tma_limit = p.total_bytes & ~(int64_t)15;
       int issued = 0;

@@ -38,6 +38,7 @@ struct DecodeRegsParams {
   int num_stages;
   int stage_stride;
   int depth;                      // copies a CTA keeps in flight (< num_stages)
+  int early_w;                    // weights are streamed before the wait for the preceding kernel
   int pre_stages;                 // stages issued before the consumers hold their activations (0 = all)
   int rows_q, rows_rem;           // n / grid, n % grid: CTA c owns rows_q (+1 if c < rows_rem) rows
   int u_begin[9];                 // unit range of k-slice s: [u_begin[s], u_begin[s+1])
@@ -446,7 +447,8 @@ __device__ __forceinline__ void decode_regs_body(const DecodeRegsParams& p, cons
   pdl_launch_dependents();
 
   if (warp == kDecodeConsumerWarps) {
-    // ---------------- producer (weights do not depend on the previous kernel: no pdl_wait before loading)
+    // ---------------- producer (with early_w the weights do not depend on the previous kernel)
+    if (!p.early_w) pdl_wait();
     if (lane == 0) {
       const int64_t tma_limit = p.total_bytes & ~(int64_t)15;
       int issued = 0;

@@ -72,7 +72,12 @@ bool supported_weight(int t) {
          t == kQ6K;
 }
 
-// launch with or without the programmatic-dependent-launch attribute
+// Every kernel goes out with the programmatic-dependent-launch attribute: all of them call griddepcontrol.wait before they
+// touch memory an earlier kernel of the stream may have written, so the attribute changes when a kernel's blocks are put on
+// the SMs, never what they see. What FUELQ_OPT_PDL adds is the caller's promise that WEIGHTS are not written by the stream's
+// preceding work, which lets a call's first kernel stream them before that wait (`early_w` of the mat-vec kernels; the later
+// kernels of a call always may: its first kernel lets them start only after its own wait, see quantize_q8k_kernel's
+// `late_trigger`).
 template <typename... KArgs, typename... Args>
 cudaError_t launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args) {
   cudaLaunchConfig_t cfg = {};
@@ -84,7 +89,7 @@ cudaError_t launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = g_opt.pdl ? 1 : 0;
+  cfg.numAttrs = 1;
   return cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...);
 }
 
@@ -99,7 +104,7 @@ int32_t quantize_act_impl(int weight_type, int64_t m, int64_t k, const float* x,
   if (!x || (!ref_out && !packed)) return kInvalidProblem;
   if (!aligned(x, 16)) return kMisaligned;
   const int64_t total = m * k;
-  const int warps_per_cta = 8;
+  const int warps_per_cta = 8, late = g_opt.pdl ? 0 : 1;
   if (at == kQ8K) {
     const int64_t nb = total / QK_K;
     const dim3 grid((unsigned)((nb + warps_per_cta - 1) / warps_per_cta)), block(32 * warps_per_cta);
@@ -107,11 +112,11 @@ int32_t quantize_act_impl(int weight_type, int64_t m, int64_t k, const float* x,
     if (ref_out) {
       if (!aligned(ref_out, 4)) return kMisaligned;
       e = launch(quantize_q8k_kernel<true>, grid, block, 0, stream, x, nb, (uint8_t*)ref_out, (int8_t*)nullptr,
-                 (float*)nullptr, (int16_t*)nullptr, zero_word, (int)early_x);
+                 (float*)nullptr, (int16_t*)nullptr, zero_word, (int)early_x, late);
     } else {
       ActPlanes a = act_planes(packed, weight_type, m, k);
       e = launch(quantize_q8k_kernel<false>, grid, block, 0, stream, x, nb, (uint8_t*)nullptr, (int8_t*)a.qs,
-                 (float*)a.d, (int16_t*)a.bsums, zero_word, (int)early_x);
+                 (float*)a.d, (int16_t*)a.bsums, zero_word, (int)early_x, late);
     }
     return e == cudaSuccess ? kOk : kLaunchFailure;
   }
@@ -123,20 +128,20 @@ int32_t quantize_act_impl(int weight_type, int64_t m, int64_t k, const float* x,
     if (ref_out) {
       if (!aligned(ref_out, 4)) return kMisaligned;
       e = launch(quantize_q8_0_kernel<true, true>, grid, block, 0, stream, x, ng, nb32, (uint8_t*)ref_out, (int8_t*)nullptr,
-                 (float*)nullptr, zero_word, (int)early_x, (float*)nullptr);
+                 (float*)nullptr, zero_word, (int)early_x, late, (float*)nullptr);
     } else {
       ActPlanes a = act_planes(packed, weight_type, m, k);
       e = launch(quantize_q8_0_kernel<false, true>, grid, block, 0, stream, x, ng, nb32, (uint8_t*)nullptr, (int8_t*)a.qs,
-                 (float*)a.d, zero_word, (int)early_x, (float*)a.bsums);
+                 (float*)a.d, zero_word, (int)early_x, late, (float*)a.bsums);
     }
   } else if (ref_out) {
     if (!aligned(ref_out, 2)) return kMisaligned;
     e = launch(quantize_q8_0_kernel<true, false>, grid, block, 0, stream, x, ng, nb32, (uint8_t*)ref_out, (int8_t*)nullptr,
-               (float*)nullptr, zero_word, (int)early_x, (float*)nullptr);
+               (float*)nullptr, zero_word, (int)early_x, late, (float*)nullptr);
   } else {
     ActPlanes a = act_planes(packed, weight_type, m, k);
     e = launch(quantize_q8_0_kernel<false, false>, grid, block, 0, stream, x, ng, nb32, (uint8_t*)nullptr, (int8_t*)a.qs,
-               (float*)a.d, zero_word, (int)early_x, (float*)nullptr);
+               (float*)a.d, zero_word, (int)early_x, late, (float*)nullptr);
   }
   return e == cudaSuccess ? kOk : kLaunchFailure;
 }
@@ -296,7 +301,7 @@ cudaError_t launch_decode_regs_peer(const DecodeRegsParams& p, const DecodeRegsP
 // *host_done is a device word that is zero when the kernel starts.
 int32_t decode_regs_impl(int type, int64_t m, int64_t n, int64_t k, const void* w, const ActPlanes& planes, float* y,
                          cudaStream_t stream, const DecodeRegsPeer* peer = nullptr, const float* x_f32 = nullptr,
-                         float* host_y = nullptr, unsigned* host_done = nullptr) {
+                         float* host_y = nullptr, unsigned* host_done = nullptr, bool early_w = false) {
   if (peer && m != 1) return kNotSupported;
   if (host_y && (peer || m != 1 || !host_done)) return kNotSupported;
   if (x_f32 && (peer || (type != kQ4K && type != kQ6K))) return kNotSupported;
@@ -328,6 +333,7 @@ int32_t decode_regs_impl(int type, int64_t m, int64_t n, int64_t k, const void* 
   p.act = planes;
   p.x_f32 = x_f32;
   p.act_smem_off = staged_off;
+  p.early_w = early_w || g_opt.pdl;
   p.host_y = host_y;
   p.host_done = host_done;
   p.y = y;
@@ -437,6 +443,7 @@ int32_t decode_tree_impl(int type, int64_t n, int64_t k, const void* w, const Ac
   p.w = (const uint8_t*)w;
   p.act = planes;
   p.x_f32 = nullptr;
+  p.early_w = g_opt.pdl != 0;
   p.host_y = nullptr;
   p.host_done = nullptr;
   p.act_smem_off = 0;
@@ -460,10 +467,11 @@ int32_t decode_tree_impl(int type, int64_t n, int64_t k, const void* w, const Ac
   return e == cudaSuccess ? kOk : kLaunchFailure;
 }
 
+// early_w: the kernel before this one belongs to the same call, so the weights may be streamed beside it
 int32_t decode_impl(int type, int64_t m, int64_t n, int64_t k, const void* w, const ActPlanes& planes, float* y,
-                    cudaStream_t stream) {
+                    cudaStream_t stream, bool early_w) {
   if (g_opt.decode_kernel != 1) {
-    const int32_t st = decode_regs_impl(type, m, n, k, w, planes, y, stream);
+    const int32_t st = decode_regs_impl(type, m, n, k, w, planes, y, stream, nullptr, nullptr, nullptr, nullptr, early_w);
     if (st != kNotSupported || g_opt.decode_kernel == 2) return st;
   }
   DeviceInfo* di;
@@ -478,6 +486,7 @@ int32_t decode_impl(int type, int64_t m, int64_t n, int64_t k, const void* w, co
   p.n = n;
   p.k = (int)k;
   p.m = (int)m;
+  p.early_w = early_w || g_opt.pdl;
   p.row_bytes = (int)(k / block_elems(type) * block_bytes(type));
   p.total_bytes = n * (int64_t)p.row_bytes;
   p.rows_per_stage = pl.rows_per_stage;
@@ -635,7 +644,7 @@ cudaError_t launch_mma_batch(const MmaBatchParams& p, dim3 grid, size_t smem, cu
 
 template <class F>
 int32_t mma_batch_fmt(int n_groups, int64_t n, int64_t k, const void* w, const ActPlanes& act, const int* offsets, int fixed_rows,
-                      const int* out_rows, float* y, bool wide, cudaStream_t stream) {
+                      const int* out_rows, float* y, bool wide, cudaStream_t stream, bool early_w) {
   DeviceInfo* di;
   if (!device_info(&di)) return kLaunchFailure;
   const int nblk = (int)(k / 256);
@@ -672,6 +681,7 @@ int32_t mma_batch_fmt(int n_groups, int64_t n, int64_t k, const void* w, const A
   p.act = act;
   p.offsets = offsets;
   p.fixed_rows = fixed_rows;
+  p.early_w = early_w || g_opt.pdl;
   p.out_rows = out_rows;
   p.y = y;
   p.n = (int)n;
@@ -704,15 +714,15 @@ int32_t mma_batch_fmt(int n_groups, int64_t n, int64_t k, const void* w, const A
 
 // kNotSupported when the format or shape has no plan here (the caller falls back)
 int32_t mma_batch_impl(int type, int n_groups, int64_t n, int64_t k, const void* w, const ActPlanes& act, const int* offsets,
-                       int fixed_rows, const int* out_rows, float* y, bool wide, cudaStream_t stream) {
+                       int fixed_rows, const int* out_rows, float* y, bool wide, cudaStream_t stream, bool early_w = false) {
   if (k % 256 || k > (1 << 20) || n > (1 << 24) || n_groups > 65535) return kNotSupported;
   switch (type) {
-    case kQ4K: return mma_batch_fmt<MbQ4K>(n_groups, n, k, w, act, offsets, fixed_rows, out_rows, y, wide, stream);
-    case kQ5K: return mma_batch_fmt<MbQ5K>(n_groups, n, k, w, act, offsets, fixed_rows, out_rows, y, wide, stream);
-    case kQ6K: return mma_batch_fmt<MbQ6K>(n_groups, n, k, w, act, offsets, fixed_rows, out_rows, y, wide, stream);
-    case kQ8_0: return mma_batch_fmt<MbQ8_0>(n_groups, n, k, w, act, offsets, fixed_rows, out_rows, y, wide, stream);
-    case kQ4_0: return mma_batch_fmt<MbQ4_0>(n_groups, n, k, w, act, offsets, fixed_rows, out_rows, y, wide, stream);
-    case kQ5_0: return mma_batch_fmt<MbQ5_0>(n_groups, n, k, w, act, offsets, fixed_rows, out_rows, y, wide, stream);
+    case kQ4K: return mma_batch_fmt<MbQ4K>(n_groups, n, k, w, act, offsets, fixed_rows, out_rows, y, wide, stream, early_w);
+    case kQ5K: return mma_batch_fmt<MbQ5K>(n_groups, n, k, w, act, offsets, fixed_rows, out_rows, y, wide, stream, early_w);
+    case kQ6K: return mma_batch_fmt<MbQ6K>(n_groups, n, k, w, act, offsets, fixed_rows, out_rows, y, wide, stream, early_w);
+    case kQ8_0: return mma_batch_fmt<MbQ8_0>(n_groups, n, k, w, act, offsets, fixed_rows, out_rows, y, wide, stream, early_w);
+    case kQ4_0: return mma_batch_fmt<MbQ4_0>(n_groups, n, k, w, act, offsets, fixed_rows, out_rows, y, wide, stream, early_w);
+    case kQ5_0: return mma_batch_fmt<MbQ5_0>(n_groups, n, k, w, act, offsets, fixed_rows, out_rows, y, wide, stream, early_w);
     default: return kNotSupported;
   }
 }
@@ -720,13 +730,13 @@ int32_t mma_batch_impl(int type, int n_groups, int64_t n, int64_t k, const void*
 // Any m_total through the decode kernels: activation rows are taken kDecodeMaxM at a time, each
 // chunk streaming the weights once. Exactly the integer arithmetic of the small-M path.
 int32_t decode_chunked(int type, int64_t m_total, int64_t n, int64_t k, const void* w, void* packed_act, float* y,
-                       cudaStream_t stream) {
+                       cudaStream_t stream, bool early_w) {
   const ActPlanes all = act_planes(packed_act, type, m_total, k);
   // (Q4_0 / Q5_0 have no register-resident one-row kernel: their single rows take this path too, measured 11.9 against
   // 14.3 us on the generic kernel for 4096 -> 11008)
   if ((m_total >= g_opt.dbg_mb_min_m || type == kQ4_0 || type == kQ5_0) && g_opt.decode_kernel == 0 && g_opt.moe_kernel == 0) {
     // a few rows: one pass over the weights on the integer tensor cores (up to 16 rows per pass)
-    const int32_t st = mma_batch_impl(type, 1, n, k, w, all, nullptr, (int)m_total, nullptr, y, m_total > 8, stream);
+    const int32_t st = mma_batch_impl(type, 1, n, k, w, all, nullptr, (int)m_total, nullptr, y, m_total > 8, stream, early_w);
     if (st != kNotSupported) return st;
   }
   // (when k is so large that the tensor-core kernel sweeps it in chunks, two-row dp4a passes stay ahead up to 5 rows)
@@ -748,7 +758,7 @@ int32_t decode_chunked(int type, int64_t m_total, int64_t n, int64_t k, const vo
     a.qs = all.qs + m0 * k;
     a.d = all.d + m0 * (k / abe);
     a.bsums = all.bsums ? all.bsums + m0 * (k / 16) : nullptr;
-    const int32_t st = decode_impl(type, mc, n, k, w, a, y + m0 * n, stream);
+    const int32_t st = decode_impl(type, mc, n, k, w, a, y + m0 * n, stream, early_w);
     if (st != kOk) return st;
   }
   return kOk;
@@ -1200,7 +1210,7 @@ int32_t fuelq_qmatmul_packed(int32_t ggml_type, int64_t m_total, int64_t n, int6
     const int32_t sp = prefetch_impl(w, n * (k / block_elems(ggml_type)) * block_bytes(ggml_type), (cudaStream_t)stream);
     if (sp != kOk) return sp;
   }
-  return decode_chunked(ggml_type, m_total, n, k, w, const_cast<void*>(packed_act), y, (cudaStream_t)stream);
+  return decode_chunked(ggml_type, m_total, n, k, w, const_cast<void*>(packed_act), y, (cudaStream_t)stream, false);
 }
 
 static int32_t qmatmul_integer(int32_t ggml_type, int64_t m_total, int64_t n, int64_t k, const void* w, const float* x,
@@ -1245,7 +1255,7 @@ static int32_t qmatmul_integer(int32_t ggml_type, int64_t m_total, int64_t n, in
   }
   st = quantize_act_impl(ggml_type, m_total, k, x, nullptr, workspace, (cudaStream_t)stream);
   if (st != kOk) return st;
-  return decode_chunked(ggml_type, m_total, n, k, w, workspace, y, (cudaStream_t)stream);
+  return decode_chunked(ggml_type, m_total, n, k, w, workspace, y, (cudaStream_t)stream, true);
 }
 
 int32_t fuelq_qmatmul_sharded(int32_t ggml_type, int64_t m_total, int64_t n_local, int64_t k, const void* w_local,
@@ -1309,10 +1319,10 @@ int32_t fuelq_qmatmul_host(int32_t ggml_type, int64_t m_total, int64_t n, int64_
       // before the mat-vec ends, and sixteen thread blocks share the copy.
       const bool wb_inside = g_opt.dbg_host_wb == 2 || (g_opt.dbg_host_wb == 0 && !g_opt.pdl);
       if (m_total == 1 && wb_inside && g_opt.decode_kernel != 1) {
-        s1 = decode_regs_impl(ggml_type, 1, n, k, w, act_planes(p, ggml_type, 1, k), y_dev, stream, nullptr, nullptr, ym, done);
+        s1 = decode_regs_impl(ggml_type, 1, n, k, w, act_planes(p, ggml_type, 1, k), y_dev, stream, nullptr, nullptr, ym, done, true);
         if (s1 != kNotSupported) return s1;
       }
-      s1 = decode_chunked(ggml_type, m_total, n, k, w, p, y_dev, stream);
+      s1 = decode_chunked(ggml_type, m_total, n, k, w, p, y_dev, stream, true);
       if (s1 != kOk) return s1;
       const long long words = (long long)m_total * n;
       const unsigned grid = (unsigned)std::min<long long>((words / 4 + 255) / 256 + 1, 16);

@@ -47,6 +47,7 @@ struct MmaBatchParams {
   int64_t group_bytes;   // n * row_bytes
   int64_t total_bytes;   // n_groups * group_bytes
   int fixed_rows;
+  int early_w;           // one group of fixed size: the weights are streamed before the wait for the preceding kernel
   int n, k, row_bytes;
   int n_wgroups;         // consumer warp groups (1, 2 or 4): group g takes stages g, g + n_wgroups, ... and its warps split k
   int num_stages, stage_stride;
@@ -597,7 +598,7 @@ __global__ void __launch_bounds__(kMbThreads, 1) mma_batch_kernel(const MmaBatch
   pdl_launch_dependents();
   // Row ranges and activations come from the preceding kernels; the weights do not, so with one group of fixed size
   // (a dense batch) the producer starts streaming before the predecessor has finished.
-  const bool early = warp == kMbConsumerWarps && !p.offsets;  // the producer of a dense batch
+  const bool early = warp == kMbConsumerWarps && !p.offsets && p.early_w;  // the producer of a dense batch
   if (!early) pdl_wait();
   const int m_begin = p.offsets ? p.offsets[grp] : 0;
   const int m_count = p.offsets ? p.offsets[grp + 1] - m_begin : p.fixed_rows;
