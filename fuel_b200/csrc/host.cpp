@@ -4,8 +4,11 @@
 
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstddef>
 #include <cstring>
+#include <map>
+#include <unordered_map>
 
 #include "../../include/fuelq.h"
 #include "../../include/fuelq_seam.h"
@@ -20,6 +23,70 @@ void cuda_check(cudaError_t e, const char* op) {
   if (e != cudaSuccess) throw Error(std::string(op) + ": " + cudaGetErrorString(e), FUELQ_LAUNCH_FAILURE);
 }
 cudaStream_t cs(const Device& d) { return static_cast<cudaStream_t>(d.stream()); }
+
+// Freed device blocks kept for the next allocation of about their size. cudaMalloc and cudaFree map and unmap memory: 0.5 to
+// 60 ms each was measured for a 9 MB matrix on a shared host, against microseconds for quantizing one, so a program that
+// converts or swaps weights spent its time there. At most kMostBytes per device are kept; what does not fit goes back to
+// the driver at once, and everything kept does when an allocation fails.
+class BlockCache {
+ public:
+  static constexpr size_t kMostBytes = (size_t)512 << 20, kGranule = (size_t)2 << 20;
+  static BlockCache& instance() {
+    static BlockCache* c = new BlockCache;  // never destroyed: buffers may be released during process exit
+    return *c;
+  }
+  // small blocks keep their size: the driver packs them into one granule
+  static size_t rounded(size_t bytes) { return bytes < kGranule / 2 ? std::max<size_t>(bytes, 16) : (bytes + kGranule - 1) / kGranule * kGranule; }
+  cudaError_t take(int ordinal, size_t bytes, void** out) {  // the device is current
+    {
+      std::lock_guard<std::mutex> lock(mu_);
+      auto& free = free_[ordinal];
+      auto it = free.lower_bound(bytes);
+      if (it != free.end() && it->first <= bytes + bytes / 8) {
+        *out = it->second;
+        kept_[ordinal] -= it->first;
+        sizes_[*out] = it->first;
+        free.erase(it);
+        return cudaSuccess;
+      }
+    }
+    cudaError_t e = cudaMalloc(out, bytes);
+    if (e == cudaErrorMemoryAllocation) {
+      cudaGetLastError();
+      flush(ordinal);
+      e = cudaMalloc(out, bytes);
+    }
+    if (e == cudaSuccess) {
+      std::lock_guard<std::mutex> lock(mu_);
+      sizes_[*out] = bytes;
+    }
+    return e;
+  }
+  void give(int ordinal, void* p) {  // the device is current; like cudaFree, waits for work that may still use the block
+    const bool idle = cudaDeviceSynchronize() == cudaSuccess;
+    std::lock_guard<std::mutex> lock(mu_);
+    const size_t bytes = sizes_[p];
+    sizes_.erase(p);
+    if (idle && kept_[ordinal] + bytes <= kMostBytes) {
+      free_[ordinal].emplace(bytes, p);
+      kept_[ordinal] += bytes;
+    } else {
+      cudaFree(p);
+    }
+  }
+
+ private:
+  void flush(int ordinal) {
+    std::lock_guard<std::mutex> lock(mu_);
+    for (auto& b : free_[ordinal]) cudaFree(b.second);
+    free_[ordinal].clear();
+    kept_[ordinal] = 0;
+  }
+  std::mutex mu_;
+  std::map<int, std::multimap<size_t, void*>> free_;
+  std::map<int, size_t> kept_;
+  std::unordered_map<void*, size_t> sizes_;
+};
 }  // namespace
 
 size_t type_size(GgmlDType t) {
@@ -57,13 +124,13 @@ void Device::synchronize() const {
 
 DeviceBuffer::DeviceBuffer(const Device& dev, size_t bytes, bool zero) : bytes_(bytes), ordinal_(dev.ordinal()) {
   dev.make_current();
-  cuda_check(cudaMalloc(&ptr_, bytes ? bytes : 16), "cudaMalloc");
+  cuda_check(BlockCache::instance().take(ordinal_, BlockCache::rounded(bytes), &ptr_), "cudaMalloc");
   if (zero && bytes) cuda_check(cudaMemsetAsync(ptr_, 0, bytes, static_cast<cudaStream_t>(dev.stream())), "cudaMemset");
 }
 DeviceBuffer::~DeviceBuffer() {
   if (ptr_) {
     cudaSetDevice(ordinal_);
-    cudaFree(ptr_);
+    BlockCache::instance().give(ordinal_, ptr_);
   }
 }
 DeviceBuffer::DeviceBuffer(DeviceBuffer&& o) noexcept : ptr_(o.ptr_), bytes_(o.bytes_), ordinal_(o.ordinal_) {
@@ -74,7 +141,7 @@ DeviceBuffer& DeviceBuffer::operator=(DeviceBuffer&& o) noexcept {
   if (this != &o) {
     if (ptr_) {
       cudaSetDevice(ordinal_);
-      cudaFree(ptr_);
+      BlockCache::instance().give(ordinal_, ptr_);
     }
     ptr_ = o.ptr_, bytes_ = o.bytes_, ordinal_ = o.ordinal_;
     o.ptr_ = nullptr, o.bytes_ = 0;
@@ -147,11 +214,20 @@ std::vector<uint8_t> QStorage::data() const {
   return out;
 }
 
-void QStorage::ensure_workspace(size_t bytes) const {
-  if (workspace_.bytes() < bytes) {
-    dev_.synchronize();  // an earlier call may still be reading the old one
-    workspace_ = DeviceBuffer(dev_, bytes, false);
-  }
+std::shared_ptr<SharedWorkspace> SharedWorkspace::of(const Device& dev) {
+  static std::mutex mu;
+  static std::map<std::pair<int, void*>, std::weak_ptr<SharedWorkspace>> all;
+  std::lock_guard<std::mutex> lock(mu);
+  for (auto it = all.begin(); it != all.end();) it = it->second.expired() ? all.erase(it) : std::next(it);
+  std::weak_ptr<SharedWorkspace>& slot = all[{dev.ordinal(), dev.stream()}];
+  std::shared_ptr<SharedWorkspace> ws = slot.lock();
+  if (!ws) slot = ws = std::make_shared<SharedWorkspace>();
+  return ws;
+}
+void* SharedWorkspace::ensure(const Device& dev, size_t need) {
+  if (bytes() < need || buffers.empty())
+    buffers.emplace_back(dev, std::max<size_t>({need, 2 * bytes(), (size_t)1 << 20}), false);
+  return buffers.back().ptr();
 }
 
 void QStorage::fwd_into(const Shape& self_shape, const float* x, const Shape& in_shape, float* y) const {
@@ -159,12 +235,16 @@ void QStorage::fwd_into(const Shape& self_shape, const float* x, const Shape& in
   const int64_t n = self_shape[0], k = self_shape[1];
   if (in_shape.size() < 2) throw Error("input tensor has only one dimension", FUELQ_INVALID_PROBLEM);
   if (in_shape.back() != k) throw Error("input tensor incompatible with the weight shape", FUELQ_INVALID_PROBLEM);
-  const int64_t m = elem_count(in_shape) / (k ? k : 1);
+  fwd_rows(n, k, x, elem_count(in_shape) / (k ? k : 1), y);
+}
+
+void QStorage::fwd_rows(int64_t n, int64_t k, const float* x, int64_t m, float* y) const {
   dev_.make_current();
   const size_t need = fuelq_qmatmul_workspace_bytes((int32_t)dtype_, m, n, k);
-  ensure_workspace(need ? need : 16);
-  check(fuelq_qmatmul((int32_t)dtype_, m, n, k, buf_.ptr(), x, y, workspace_.ptr(), workspace_.bytes(), dev_.stream()),
-        "fuelq_qmatmul");
+  SharedWorkspace& ws = *workspace_;
+  std::lock_guard<std::mutex> lock(ws.mutex);
+  void* scratch = ws.ensure(dev_, need);
+  check(fuelq_qmatmul((int32_t)dtype_, m, n, k, buf_.ptr(), x, y, scratch, ws.bytes(), dev_.stream()), "fuelq_qmatmul");
 }
 
 std::pair<DeviceBuffer, Shape> QStorage::fwd(const Shape& self_shape, const float* x, const Shape& in_shape) const {
@@ -330,7 +410,7 @@ int32_t fuelq_qmatmul_forward(const void* h, const float* device_x, int64_t m, f
   return guarded([&] {
     if (!h) throw Error("null handle", FUELQ_INVALID_PROBLEM);
     const QTensor& t = *static_cast<const QTensorHandle*>(h)->t;
-    t.storage().fwd_into(t.shape(), device_x, Shape{m, t.shape()[1]}, device_y);
+    t.storage().fwd_rows(t.shape()[0], t.shape()[1], device_x, m, device_y);
   });
 }
 

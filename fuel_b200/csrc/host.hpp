@@ -15,6 +15,7 @@
 #include <cstddef>
 #include <cstdint>
 #include <memory>
+#include <mutex>
 #include <stdexcept>
 #include <string>
 #include <vector>
@@ -77,6 +78,20 @@ class DeviceBuffer {
   int ordinal_ = 0;
 };
 
+// Device scratch for fwd, shared by every storage on one (device, stream): the calls of a stream run in order, so one buffer
+// serves all of a model's linears (one each would cost a model of two hundred of them gigabytes, and an allocation with a
+// device synchronization on each one's first call). Growing keeps the smaller buffers, since kernels in flight or captured
+// graphs may hold their addresses; growth is at least twofold, so the total stays below twice the largest need, and all of
+// it is released with the last storage that uses it. A caller holds `mutex` while it enqueues the kernels of one product, so
+// that two threads on one stream do not interleave theirs.
+struct SharedWorkspace {
+  std::mutex mutex;
+  std::vector<DeviceBuffer> buffers;  // the last one is the largest
+  static std::shared_ptr<SharedWorkspace> of(const Device& dev);
+  void* ensure(const Device& dev, size_t bytes);  // with `mutex` held
+  size_t bytes() const { return buffers.empty() ? 0 : buffers.back().bytes(); }
+};
+
 class QStorage {
  public:
   // QCudaStorage::zeros, fuel-cuda-backend/src/quantized.rs:307-320
@@ -109,15 +124,17 @@ class QStorage {
   std::pair<DeviceBuffer, Shape> fwd(const Shape& self_shape, const float* device_input, const Shape& input_shape) const;
   // same, into caller-owned output (what a graph executor with pre-allocated outputs calls)
   void fwd_into(const Shape& self_shape, const float* device_input, const Shape& input_shape, float* device_out) const;
+  // the same for an input already known to be [m, k] against [n, k]
+  void fwd_rows(int64_t n, int64_t k, const float* device_input, int64_t m, float* device_out) const;
 
  private:
-  QStorage(const Device& dev, GgmlDType dtype, size_t len) : dev_(dev), dtype_(dtype), len_(len) {}
-  void ensure_workspace(size_t bytes) const;
+  QStorage(const Device& dev, GgmlDType dtype, size_t len)
+      : dev_(dev), dtype_(dtype), len_(len), workspace_(SharedWorkspace::of(dev)) {}
   Device dev_;
   GgmlDType dtype_;
   size_t len_ = 0;
   DeviceBuffer buf_;
-  mutable DeviceBuffer workspace_;  // activation blocks for fwd; grown on demand, reused across calls
+  std::shared_ptr<SharedWorkspace> workspace_;
 };
 
 class QTensor {

@@ -535,7 +535,7 @@ class QLlama:
         stamped stores inside the kernels; otherwise through the library's all-gather (nothing travels on one GPU).
         Norm, attention merge and SwiGLU write the next mat-vec's quantized activations directly."""
         c, r, g = self.cfg, self.rank, self.world
-        st = torch.cuda.current_stream().cuda_stream
+        st = torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
         scale = 1.0 / math.sqrt(c.head_dim)
         pk, pkn = self.packed.data_ptr(), self.packed.numel()
         fl = self.f_hi - self.f_lo
@@ -600,7 +600,7 @@ class QLlama:
     def _step_plain(self) -> None:
         """One GPU, any supported linear formats: every op its own call, activations quantized per consumer."""
         c = self.cfg
-        st = torch.cuda.current_stream().cuda_stream
+        st = torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
         scale = 1.0 / math.sqrt(c.head_dim)
         fl = c.ffn_dim
         _check(_L.fuelq_embed_rows(int(self.embed_dtype), self.embed.data_ptr(), c.dim, self.token.data_ptr(), 1, self.x.data_ptr(), st),

@@ -14,6 +14,7 @@ from . import _lib
 from .ggml import GgmlDType as T
 
 _L = _lib.lib
+_raw_stream = torch._C._cuda_getCurrentRawStream   # the handle alone: a Stream object costs microseconds
 
 
 def _check(st: int, op: str) -> None:
@@ -53,7 +54,7 @@ class QMoeBlock:
         assert self.first == 0 and self.E == self.E_total, "use the expert-parallel driver for a partial expert set"
         if out is None:
             out = torch.empty(n, self.H, dtype=torch.float32, device=self.device)
-        st = torch.cuda.current_stream().cuda_stream
+        st = _raw_stream(torch.cuda.current_device())
         P = n * self.K
         _check(_L.fuelq_moe_route(logits.data_ptr(), n, self.E_total, self.K, self.topk_ids.data_ptr(),
                                   self.topk_w.data_ptr(), st), "fuelq_moe_route")
@@ -121,7 +122,7 @@ class QMoeExpertParallel:
         n = x.shape[0]
         P = n * self.K
         assert P <= C
-        st = torch.cuda.current_stream().cuda_stream
+        st = _raw_stream(torch.cuda.current_device())
         _check(_L.fuelq_moe_route(logits.data_ptr(), n, self.E, self.K, h.topk_ids.data_ptr(), h.topk_w.data_ptr(), st),
                "fuelq_moe_route")
         _check(_L.fuelq_moe_bucket(h.topk_ids.data_ptr(), P, self.E, h.sorted_ids.data_ptr(), h.offsets.data_ptr(), st),

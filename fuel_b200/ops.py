@@ -12,11 +12,12 @@ from . import _lib
 from .ggml import GgmlDType
 
 _L = _lib.lib
+_raw_stream = torch._C._cuda_getCurrentRawStream   # the handle alone: a Stream object costs microseconds
 _OUT_TYPES = {torch.float32: GgmlDType.F32, torch.float16: GgmlDType.F16, torch.bfloat16: GgmlDType.BF16}
 
 
 def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    return _raw_stream(torch.cuda.current_device())
 
 
 def _need_cuda(t: torch.Tensor, name: str) -> None:

@@ -17,6 +17,9 @@ from . import _lib
 from .ggml import GgmlDType
 
 _L = _lib.lib
+_forward = _L.fuelq_qmatmul_forward
+_current_device = torch.cuda.current_device
+_raw_stream = torch._C._cuda_getCurrentRawStream   # the handle alone: a Stream object costs microseconds
 _OUT_TYPES = {torch.float32: GgmlDType.F32, torch.float16: GgmlDType.F16, torch.bfloat16: GgmlDType.BF16}
 
 
@@ -30,7 +33,7 @@ class QTensor:
 
     def __init__(self, handle: int, device: torch.device):
         self._h = ctypes.c_void_p(handle)
-        self.device = device
+        self.device, self._index = device, device.index
         t, n, k, nbytes, ptr = ctypes.c_int32(), ctypes.c_int64(), ctypes.c_int64(), ctypes.c_size_t(), ctypes.c_void_p()
         _check(_L.fuelq_qtensor_info(self._h, ctypes.byref(t), ctypes.byref(n), ctypes.byref(k), ctypes.byref(nbytes),
                                      ctypes.byref(ptr)), "qtensor_info")
@@ -62,7 +65,7 @@ class QTensor:
             ptr, on_dev = src.ctypes.data, 0
         out = ctypes.c_void_p()
         with torch.cuda.device(idx):
-            stream = torch.cuda.current_stream().cuda_stream
+            stream = _raw_stream(idx)
             _check(_L.fuelq_qtensor_quantize(idx, stream, int(dtype), n, k, ptr, on_dev, ctypes.byref(out)), "QTensor.quantize")
             torch.cuda.current_stream().synchronize()
         return cls(out.value, torch.device("cuda", idx))
@@ -76,7 +79,7 @@ class QTensor:
         n, k = shape
         out = ctypes.c_void_p()
         with torch.cuda.device(idx):
-            stream = torch.cuda.current_stream().cuda_stream
+            stream = _raw_stream(idx)
             _check(_L.fuelq_qtensor_load(idx, stream, int(dtype), n, k, blocks.ctypes.data, blocks.size, ctypes.byref(out)),
                    "QTensor.from_blocks")
         return cls(out.value, torch.device("cuda", idx))
@@ -137,17 +140,24 @@ class QMatMul:
             with torch.cuda.device(self.w.device):
                 _check(_L.fuelq_qmatmul_forward_host(self.w._h, x.ctypes.data, x.size // k, y.ctypes.data), "QMatMul.forward")
             return torch.from_numpy(y) if isinstance(xs, torch.Tensor) else y
+        w = self.w
         if xs.dtype != torch.float32:
             raise _lib.FuelqError("QMatMul.forward", _lib.NOT_SUPPORTED, "Expected f32")
         if not xs.is_contiguous():
             raise _lib.FuelqError("QMatMul.forward", _lib.INVALID_PROBLEM, "input tensor is not contiguous")
         if xs.dim() < 2:
             raise _lib.FuelqError("QMatMul.forward", _lib.INVALID_PROBLEM, "input tensor has only one dimension")
-        if xs.shape[-1] != k:
+        shape = xs.shape
+        if shape[-1] != k:
             raise _lib.FuelqError("QMatMul.forward", _lib.INVALID_PROBLEM, "input tensor incompatible with the weight shape")
-        y = torch.empty(*xs.shape[:-1], n, dtype=torch.float32, device=xs.device)
-        with torch.cuda.device(xs.device):
-            _check(_L.fuelq_qmatmul_forward(self.w._h, xs.data_ptr(), xs.numel() // k, y.data_ptr()), "QMatMul.forward")
+        y = xs.new_empty((*shape[:-1], n))
+        if w.device == xs.device and w._index == _current_device():   # the usual case: no device to switch to and back
+            status = _forward(w._h, xs.data_ptr(), xs.numel() // k, y.data_ptr())
+        else:
+            with torch.cuda.device(xs.device):
+                status = _forward(w._h, xs.data_ptr(), xs.numel() // k, y.data_ptr())
+        if status:
+            _check(status, "QMatMul.forward")
         return y
 
     __call__ = forward
