@@ -6,14 +6,15 @@
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
+#include <cmath>
+
 #include "decode.cuh"
 #include "decode_regs.cuh"
 #include "dequantize.cuh"
 #include "fq_common.cuh"
+#include "ibatch.cuh"
 #include "llama_glue.cuh"
-#include "mma_batch.cuh"
 #include "moe.cuh"
-#include "moe_mma.cuh"
 #include "plain_gemm.cuh"
 #include "prefill.cuh"
 #include "quantize_act.cuh"
@@ -37,7 +38,7 @@ struct Options {
   int64_t prefill_tf32 = 0;   // tensor-core path in tf32 instead of 16-bit operands
   int64_t prefill_bf16 = 0;   // 16-bit operands as bf16 instead of f16
   int64_t fused_quant = 0;    // f32 activations with m <= 2: quantize inside the mat-vec kernel
-  int64_t dbg_mb_groups = 0, dbg_mb_min_m = 2, dbg_mb_rpc = 0;
+  int64_t dbg_ib_waves = 0;    // grouped matmul: thread blocks per SM in all
   int64_t dbg_host_wb = 0;     // write-back to a host buffer: 0 = by launch mode, 1 = own kernel, 2 = inside the mat-vec kernel
   int64_t dbg_host_early = 1;  // host activations loaded before the wait for earlier kernels
   int64_t dbg_slab_kb = 0;     // tensor-core path through dequantized slabs: slab size in KiB (0 = 128 MiB)
@@ -94,8 +95,9 @@ cudaError_t launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
 }
 
 // ------------------------------------------------------------------ activation quantization
+// `planes`: the plane layout whatever the row count (the kernels selected by the kernel options read nothing else)
 int32_t quantize_act_impl(int weight_type, int64_t m, int64_t k, const float* x, void* ref_out, void* packed,
-                          cudaStream_t stream, unsigned* zero_word = nullptr, bool early_x = false) {
+                          cudaStream_t stream, bool planes = false, unsigned* zero_word = nullptr, bool early_x = false) {
   if (!supported_weight(weight_type)) return kNotSupported;
   const int at = act_type_for(weight_type);
   const int be = block_elems(at);
@@ -104,6 +106,8 @@ int32_t quantize_act_impl(int weight_type, int64_t m, int64_t k, const float* x,
   if (!x || (!ref_out && !packed)) return kInvalidProblem;
   if (!aligned(x, 16)) return kMisaligned;
   const int64_t total = m * k;
+  uint8_t* rec = packed && !planes && act_records(m, k) ? (uint8_t*)packed : nullptr;
+  const int rows = (int)m, nblk = (int)(k / QK_K);
   const int warps_per_cta = 8, late = g_opt.pdl ? 0 : 1;
   if (at == kQ8K) {
     const int64_t nb = total / QK_K;
@@ -112,11 +116,11 @@ int32_t quantize_act_impl(int weight_type, int64_t m, int64_t k, const float* x,
     if (ref_out) {
       if (!aligned(ref_out, 4)) return kMisaligned;
       e = launch(quantize_q8k_kernel<true>, grid, block, 0, stream, x, nb, (uint8_t*)ref_out, (int8_t*)nullptr,
-                 (float*)nullptr, (int16_t*)nullptr, zero_word, (int)early_x, late);
+                 (float*)nullptr, (int16_t*)nullptr, (uint8_t*)nullptr, rows, nblk, zero_word, (int)early_x, late);
     } else {
       ActPlanes a = act_planes(packed, weight_type, m, k);
       e = launch(quantize_q8k_kernel<false>, grid, block, 0, stream, x, nb, (uint8_t*)nullptr, (int8_t*)a.qs,
-                 (float*)a.d, (int16_t*)a.bsums, zero_word, (int)early_x, late);
+                 (float*)a.d, (int16_t*)a.bsums, rec, rows, nblk, zero_word, (int)early_x, late);
     }
     return e == cudaSuccess ? kOk : kLaunchFailure;
   }
@@ -128,20 +132,20 @@ int32_t quantize_act_impl(int weight_type, int64_t m, int64_t k, const float* x,
     if (ref_out) {
       if (!aligned(ref_out, 4)) return kMisaligned;
       e = launch(quantize_q8_0_kernel<true, true>, grid, block, 0, stream, x, ng, nb32, (uint8_t*)ref_out, (int8_t*)nullptr,
-                 (float*)nullptr, zero_word, (int)early_x, late, (float*)nullptr);
+                 (float*)nullptr, (uint8_t*)nullptr, rows, nblk, zero_word, (int)early_x, late, (float*)nullptr);
     } else {
       ActPlanes a = act_planes(packed, weight_type, m, k);
       e = launch(quantize_q8_0_kernel<false, true>, grid, block, 0, stream, x, ng, nb32, (uint8_t*)nullptr, (int8_t*)a.qs,
-                 (float*)a.d, zero_word, (int)early_x, late, (float*)a.bsums);
+                 (float*)a.d, rec, rows, nblk, zero_word, (int)early_x, late, (float*)a.bsums);
     }
   } else if (ref_out) {
     if (!aligned(ref_out, 2)) return kMisaligned;
     e = launch(quantize_q8_0_kernel<true, false>, grid, block, 0, stream, x, ng, nb32, (uint8_t*)ref_out, (int8_t*)nullptr,
-               (float*)nullptr, zero_word, (int)early_x, late, (float*)nullptr);
+               (float*)nullptr, (uint8_t*)nullptr, rows, nblk, zero_word, (int)early_x, late, (float*)nullptr);
   } else {
     ActPlanes a = act_planes(packed, weight_type, m, k);
     e = launch(quantize_q8_0_kernel<false, false>, grid, block, 0, stream, x, ng, nb32, (uint8_t*)nullptr, (int8_t*)a.qs,
-               (float*)a.d, zero_word, (int)early_x, late, (float*)nullptr);
+               (float*)a.d, rec, rows, nblk, zero_word, (int)early_x, late, (float*)nullptr);
   }
   return e == cudaSuccess ? kOk : kLaunchFailure;
 }
@@ -561,74 +565,11 @@ int32_t prefetch_impl(const void* w, int64_t bytes, cudaStream_t stream) {
   return e == cudaSuccess ? kOk : kLaunchFailure;
 }
 
-// Tensor-core form (Q4_K): kNotSupported when the shared-memory plan does not fit, so the caller can fall back.
-int32_t moe_mma_impl(int n_groups, int64_t n, int64_t k, const void* w, const ActPlanes& act, const int* offsets,
-                     int fixed_rows, const int* out_rows, float* y, cudaStream_t stream) {
-  DeviceInfo* di;
-  if (!device_info(&di)) return kLaunchFailure;
-  MmaParams p;
-  p.row_bytes = (int)(k / 256 * Q4KL::kBytes);
-  const size_t header = align_up(sizeof(MmaSmemHeader), 128);
-  const size_t per_cta = ((size_t)di->max_smem_optin + 1024) / 2 - 1024 - 512;
-  const size_t part_bytes = kDecodeConsumerWarps * 128 * sizeof(float);
-  // k in as few chunks as shared memory allows: one chunk of the activation rows plus two stages of eight weight rows
-  const int nblk = (int)(k / 256);
-  int R = 0, kc_blocks = 0;
-  size_t stride = 0, act_bytes = 0, ring = 0;
-  for (int chunks = 1; chunks <= 16 && !R; ++chunks) {
-    const int kc = (nblk + chunks - 1) / chunks;
-    const size_t ab = mma_act_bytes(kc);
-    if (header + ab + part_bytes >= per_cta) continue;
-    const size_t rg = per_cta - header - ab - part_bytes;
-    for (int cand = 32; cand >= 8; cand >>= 1) {
-      const size_t st = align_up((size_t)cand * (kc * Q4KL::kBytes + 16), 128);
-      if (2 * st <= rg) {
-        R = cand, stride = st, kc_blocks = kc, act_bytes = ab, ring = rg;
-        break;
-      }
-    }
-  }
-  if (!R) return kNotSupported;
-  int stages = (int)(ring / stride);
-  if (stages > 4) stages = 4;
-  p.w = (const uint8_t*)w;
-  p.act = act;
-  p.offsets = offsets;
-  p.fixed_rows = fixed_rows;
-  p.out_rows = out_rows;
-  p.y = y;
-  p.n = (int)n;
-  p.k = (int)k;
-  p.group_bytes = n * (int64_t)p.row_bytes;
-  p.rows_per_stage = R;
-  p.num_stages = stages;
-  p.stage_stride = (int)stride;
-  p.act_off = (int)(header + (size_t)stages * stride);
-  p.part_off = (int)(p.act_off + act_bytes);
-  p.kc_blocks = kc_blocks;
-  int per_group = ((kc_blocks < nblk ? 2 : 4) * di->sm_count + n_groups - 1) / n_groups;
-  const int max_per = (int)((n + R - 1) / R);
-  if (per_group > max_per) per_group = max_per;
-  if (per_group < 1) per_group = 1;
-  static bool attr_set[64] = {};
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (dev < 0 || dev >= 64) return kLaunchFailure;
-  if (!attr_set[dev]) {
-    if (cudaFuncSetAttribute(mma_q4k_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, di->max_smem_optin) != cudaSuccess)
-      return kLaunchFailure;
-    attr_set[dev] = true;
-  }
-  const size_t smem = header + (size_t)stages * stride + act_bytes + part_bytes;
-  const cudaError_t e = launch(mma_q4k_kernel, dim3((unsigned)per_group, (unsigned)n_groups), dim3(kDecodeThreads), smem, stream, p);
-  return e == cudaSuccess ? kOk : kLaunchFailure;
-}
-
-// ---- small batches on the integer tensor cores (mma_batch.cuh): Q4_K, Q5_K, Q6_K, Q8_0; k a multiple of 256
+// ---- a few to a few dozen rows on the integer tensor cores (ibatch.cuh): every format, k a multiple of 256
 template <class F, int MT>
-cudaError_t launch_mma_batch(const MmaBatchParams& p, dim3 grid, size_t smem, cudaStream_t stream) {
+cudaError_t launch_ibatch(const IbParams& p, dim3 grid, int warps, size_t smem, cudaStream_t stream) {
   static bool attr_set[64] = {};
-  auto kern = mma_batch_kernel<F, MT>;
+  auto kern = ibatch_kernel<F, MT>;
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
@@ -639,113 +580,135 @@ cudaError_t launch_mma_batch(const MmaBatchParams& p, dim3 grid, size_t smem, cu
     if (e != cudaSuccess) return e;
     attr_set[dev] = true;
   }
-  return launch(kern, grid, dim3(kMbThreads), smem, stream, p);
+  return launch(kern, grid, dim3(32 * warps), smem, stream, p);
+}
+
+// Shared-memory plan for `tiles` 16-row tiles per thread block of `warps` warps. The split of the warps over tiles and k is
+// the one with the fewest steps (one block of one tile each) on a warp's critical path.
+template <class F>
+bool plan_ibatch(IbParams* p, int tiles, int warps, size_t budget, size_t* smem) {
+  const int part_bytes = warps * (p->rows_cap > 8 ? 256 : 128) * 4;
+  int best = 0, best_kp = 1, best_tg = 1;
+  for (int r = (tiles + warps - 1) / warps; r <= (tiles + warps - 1) / warps + 3; ++r) {
+    const int tg = (tiles + r - 1) / r;
+    int kp = warps / tg;
+    if (kp > p->nblk) kp = p->nblk;
+    const int steps = r * ((p->nblk + kp - 1) / kp);
+    if (!best || steps < best) best = steps, best_kp = kp, best_tg = tg;
+  }
+  for (int kp = best_kp; kp >= 1; kp = kp > 4 ? kp / 2 : kp - 1) {  // fewer shares when their activations do not fit
+    const int share = (p->nblk + kp - 1) / kp, slot = p->rows_cap * ib_rec(F::kAct);
+    for (int stages = 4; stages >= 2; --stages) {
+      const size_t weights = (size_t)warps * stages * 16 * F::kPitch + (kp > 1 ? part_bytes : 0) + kIbHeader + 256;
+      if (weights >= budget) continue;
+      const size_t room = budget - weights;
+      int bpc = share, bufs = 1;
+      if ((size_t)kp * share * slot > room) {
+        if (stages == 4) continue;  // two activation buffers before a fourth weight stage
+        bpc = (int)(room / ((size_t)2 * kp * slot)), bufs = 2;
+        if (bpc < 1 || (bpc < 2 && stages > 2)) continue;
+        const int chunks = (share + bpc - 1) / bpc;
+        bpc = (share + chunks - 1) / chunks;  // even chunks
+      }
+      p->kp = kp, p->share_q = p->nblk / kp, p->share_rem = p->nblk % kp, p->tg = best_tg, p->bpc = bpc, p->n_chunks = (share + bpc - 1) / bpc, p->stages = stages;
+      p->act_off = (int)align_up(kIbHeader + (size_t)warps * stages * 16 * F::kPitch + 16, 128);
+      p->act_buf = (int)align_up((size_t)kp * bpc * slot, 128);
+      p->part_off = p->act_off + bufs * p->act_buf;
+      *smem = (size_t)p->part_off + (kp > 1 ? part_bytes : 0);
+      if (*smem <= budget) return true;
+    }
+  }
+  return false;
 }
 
 template <class F>
-int32_t mma_batch_fmt(int n_groups, int64_t n, int64_t k, const void* w, const ActPlanes& act, const int* offsets, int fixed_rows,
-                      const int* out_rows, float* y, bool wide, cudaStream_t stream, bool early_w) {
+int32_t ibatch_fmt(int n_groups, int64_t n, int64_t k, const void* w, const ActPlanes& act, const int* offsets, int64_t n_rows,
+                   const int* out_rows, float* y, cudaStream_t stream, bool early_w) {
   DeviceInfo* di;
   if (!device_info(&di)) return kLaunchFailure;
-  const int nblk = (int)(k / 256);
-  const int act_rows = wide ? 16 : 8;
-  const size_t header = align_up(sizeof(MmaBatchHeader), 128);
-  const size_t part_bytes = (size_t)kMbConsumerWarps * (wide ? 2 : 1) * 128 * sizeof(float);
-  const size_t total = (size_t)di->max_smem_optin;
-  // k in as few sweeps as shared memory allows: the activation rows of one sweep plus at least two (preferably four) stages of 16 weight rows
-  MmaBatchParams p;
-  const int R = 16;
-  int kc_blocks = 0, stages = 0;
-  size_t stride = 0, act_bytes = 0;
-  int wstride = 0;
-  // fewest sweeps over k first; within that, at least three stages (two at the very least)
-  int rpc = 1;
-  for (int chunks = 1; chunks <= 64 && !kc_blocks; ++chunks) {
-    const int kc = (nblk + chunks - 1) / chunks;
-    const size_t ab = (size_t)mb_act_layout<F>(kc, act_rows).bytes;
-    // whole rows staged: consecutive rows travel in one bulk copy (2 per copy; 4 for short rows)
-    rpc = chunks == 1 ? (g_opt.dbg_mb_rpc ? (int)g_opt.dbg_mb_rpc : (nblk * F::kBytes256 <= 1536 ? 4 : 2)) : 1;
-    // a staged copy: its bytes widened to 16-byte boundaries, placed so that consecutive copies are 16 bytes apart modulo 128
-    const int ws = (int)align_up((size_t)(rpc - 1) * nblk * F::kBytes256 + (size_t)kc * F::kBytes256 + 32, 128) + 16;
-    const size_t st = align_up((size_t)(R / rpc) * ws, 128);
-    const int min_stages = chunks < 4 ? 3 : 2;
-    if (header + ab + part_bytes + (size_t)min_stages * st <= total) {
-      kc_blocks = kc, act_bytes = ab, wstride = ws, stride = st;
-      stages = (int)((total - header - ab - part_bytes) / st);
-    }
-  }
-  if (!kc_blocks) return kNotSupported;
-  if (stages > kMbMaxStages) stages = kMbMaxStages;
-  if (g_opt.dbg_max_stages && stages > g_opt.dbg_max_stages) stages = (int)g_opt.dbg_max_stages;
+  IbParams p;
   p.w = (const uint8_t*)w;
   p.act = act;
   p.offsets = offsets;
-  p.fixed_rows = fixed_rows;
+  p.fixed_rows = (int)n_rows;
+  p.act_rows = n_rows;
   p.early_w = early_w || g_opt.pdl;
   p.out_rows = out_rows;
   p.y = y;
   p.n = (int)n;
-  p.k = (int)k;
-  p.row_bytes = nblk * F::kBytes256;
+  p.nblk = (int)(k / 256);
+  p.row_bytes = p.nblk * F::kBytes256;
   p.group_bytes = n * (int64_t)p.row_bytes;
   p.total_bytes = (int64_t)n_groups * p.group_bytes;
-  p.num_stages = stages;
-  // (never more groups than stages: a group must not wait for a slot's next phase before the slot's first use)
-  p.n_wgroups = stages >= 4 ? 4 : stages >= 2 ? 2 : 1;
-  if (g_opt.dbg_mb_groups && g_opt.dbg_mb_groups <= p.n_wgroups) p.n_wgroups = (int)g_opt.dbg_mb_groups;
-  p.stage_stride = (int)stride;
-  p.wstride = wstride;
-  p.rows_per_copy = rpc;
-  p.act_off = (int)(header + (size_t)stages * stride);
-  p.part_off = (int)(p.act_off + act_bytes);
-  p.kc_blocks = kc_blocks;
   const int n_tiles = (int)((n + 15) / 16);
-  int per_group = (di->sm_count + n_groups - 1) / n_groups;
-  if (n_groups > 1) per_group = (2 * di->sm_count + n_groups - 1) / n_groups;
+  int warps = kIbMaxWarps, per_group;
+  size_t budget = (size_t)di->max_smem_optin, smem = 0;
+  if (!offsets) {
+    p.rows_cap = n_rows >= kIbMaxRows ? kIbMaxRows : (int)((n_rows + 7) & ~7ll);
+    per_group = di->sm_count;
+    if (p.rows_cap > 32) warps = kIbMaxWarps / 2;  // twice the registers a thread
+  } else {
+    // Routed rows: enough rows per pass for most groups (their mean and twice its root), two thread blocks of eight warps
+    // per SM, so that one computes while the other stages; several blocks per group, as few groups may have rows.
+    const double mean = (double)n_rows / n_groups;
+    int cap = ((int)(mean + 2.0 * sqrt(mean)) + 8) & ~7;
+    p.rows_cap = cap < 8 ? 8 : cap > kIbMaxRows ? kIbMaxRows : cap;
+    warps = kIbMaxWarps / 2;
+    budget = ((size_t)di->max_smem_optin + 1024) / 2 - 1024;
+    const int64_t live = n_rows < n_groups ? n_rows : n_groups;
+    per_group = (int)((int64_t)(g_opt.dbg_ib_waves ? g_opt.dbg_ib_waves : 4) * di->sm_count / live) + 1;
+  }
   if (g_opt.decode_grid > 0) per_group = (int)g_opt.decode_grid;
-  const int max_per = n_tiles;
-  if (per_group > max_per) per_group = max_per;
+  if (per_group > n_tiles) per_group = n_tiles;
   if (per_group < 1) per_group = 1;
-  const size_t smem = header + (size_t)stages * stride + act_bytes + part_bytes;
+  const int tiles = (n_tiles + per_group - 1) / per_group;
+  if (!plan_ibatch<F>(&p, tiles, warps, budget, &smem)) {
+    if (!offsets) return kNotSupported;
+    if (!plan_ibatch<F>(&p, tiles, warps, (size_t)di->max_smem_optin, &smem)) return kNotSupported;
+  }
   const dim3 grid((unsigned)per_group, (unsigned)n_groups);
-  const cudaError_t e = wide ? launch_mma_batch<F, 2>(p, grid, smem, stream) : launch_mma_batch<F, 1>(p, grid, smem, stream);
+  cudaError_t e;
+  if (p.rows_cap <= 8) e = launch_ibatch<F, 1>(p, grid, warps, smem, stream);
+  else if (p.rows_cap <= 16) e = launch_ibatch<F, 2>(p, grid, warps, smem, stream);
+  else if (p.rows_cap <= 32) e = launch_ibatch<F, 4>(p, grid, warps, smem, stream);
+  else e = launch_ibatch<F, 8>(p, grid, warps, smem, stream);
   return e == cudaSuccess ? kOk : kLaunchFailure;
 }
 
-// kNotSupported when the format or shape has no plan here (the caller falls back)
-int32_t mma_batch_impl(int type, int n_groups, int64_t n, int64_t k, const void* w, const ActPlanes& act, const int* offsets,
-                       int fixed_rows, const int* out_rows, float* y, bool wide, cudaStream_t stream, bool early_w = false) {
-  if (k % 256 || k > (1 << 20) || n > (1 << 24) || n_groups > 65535) return kNotSupported;
+// kNotSupported when the shape has no plan here (the caller falls back)
+int32_t ibatch_impl(int type, int n_groups, int64_t n, int64_t k, const void* w, const ActPlanes& act, const int* offsets,
+                    int64_t n_rows, const int* out_rows, float* y, cudaStream_t stream, bool early_w) {
+  if (k % 256 || n > INT32_MAX - 64 || n_groups > 65535 || n_rows > (1 << 28)) return kNotSupported;
+#define FQ_IB(T, F) \
+  case T: return ibatch_fmt<F>(n_groups, n, k, w, act, offsets, n_rows, out_rows, y, stream, early_w)
   switch (type) {
-    case kQ4K: return mma_batch_fmt<MbQ4K>(n_groups, n, k, w, act, offsets, fixed_rows, out_rows, y, wide, stream, early_w);
-    case kQ5K: return mma_batch_fmt<MbQ5K>(n_groups, n, k, w, act, offsets, fixed_rows, out_rows, y, wide, stream, early_w);
-    case kQ6K: return mma_batch_fmt<MbQ6K>(n_groups, n, k, w, act, offsets, fixed_rows, out_rows, y, wide, stream, early_w);
-    case kQ8_0: return mma_batch_fmt<MbQ8_0>(n_groups, n, k, w, act, offsets, fixed_rows, out_rows, y, wide, stream, early_w);
-    case kQ4_0: return mma_batch_fmt<MbQ4_0>(n_groups, n, k, w, act, offsets, fixed_rows, out_rows, y, wide, stream, early_w);
-    case kQ5_0: return mma_batch_fmt<MbQ5_0>(n_groups, n, k, w, act, offsets, fixed_rows, out_rows, y, wide, stream, early_w);
+    FQ_IB(kQ4K, IbQ4K);
+    FQ_IB(kQ5K, IbQ5K);
+    FQ_IB(kQ6K, IbQ6K);
+    FQ_IB(kQ8_0, IbQ8_0);
+    FQ_IB(kQ2K, IbQ2K);
+    FQ_IB(kQ3K, IbQ3K);
+    FQ_IB(kQ4_0, IbQ4_0);
+    FQ_IB(kQ4_1, IbQ4_1);
+    FQ_IB(kQ5_0, IbQ5_0);
+    FQ_IB(kQ5_1, IbQ5_1);
     default: return kNotSupported;
   }
+#undef FQ_IB
 }
+
+bool integer_kernel_forced() { return g_opt.decode_kernel != 0 || g_opt.moe_kernel != 0; }
 
 // Any m_total through the decode kernels: activation rows are taken kDecodeMaxM at a time, each
 // chunk streaming the weights once. Exactly the integer arithmetic of the small-M path.
 int32_t decode_chunked(int type, int64_t m_total, int64_t n, int64_t k, const void* w, void* packed_act, float* y,
-                       cudaStream_t stream, bool early_w) {
-  const ActPlanes all = act_planes(packed_act, type, m_total, k);
-  // (Q4_0 / Q5_0 have no register-resident one-row kernel: their single rows take this path too, measured 11.9 against
-  // 14.3 us on the generic kernel for 4096 -> 11008)
-  if ((m_total >= g_opt.dbg_mb_min_m || type == kQ4_0 || type == kQ5_0) && g_opt.decode_kernel == 0 && g_opt.moe_kernel == 0) {
-    // a few rows: one pass over the weights on the integer tensor cores (up to 16 rows per pass)
-    const int32_t st = mma_batch_impl(type, 1, n, k, w, all, nullptr, (int)m_total, nullptr, y, m_total > 8, stream, early_w);
-    if (st != kNotSupported) return st;
-  }
-  // (when k is so large that the tensor-core kernel sweeps it in chunks, two-row dp4a passes stay ahead up to 5 rows)
-  const bool mma_chunked = k / 256 > 16;
-  if (type == kQ4K && m_total > (mma_chunked ? 5 : 2) && g_opt.decode_kernel == 0 && g_opt.moe_kernel != 1 && n <= (1 << 24)) {
-    // a few rows of Q4_K: one pass over the weights on the integer tensor cores (16 rows per pass)
-    const int32_t st = moe_mma_impl(1, n, k, w, all, nullptr, (int)m_total, nullptr, y, stream);
-    if (st != kNotSupported) return st;
-  }
+                       cudaStream_t stream, bool early_w, bool planes = false) {
+  const ActPlanes all = planes ? act_planes(packed_act, type, m_total, k) : act_layout(packed_act, type, m_total, k);
+  // One pass over the weights on the integer tensor cores (up to 64 rows per pass) from two rows up; single rows of the
+  // formats without a register-resident one-row kernel too.
+  const bool one_row_kernel = type == kQ4K || type == kQ5K || type == kQ6K || type == kQ8_0;
+  if (all.rec || (m_total == 1 && !one_row_kernel && k % 256 == 0 && !integer_kernel_forced()))
+    return ibatch_impl(type, 1, n, k, w, all, nullptr, m_total, nullptr, y, stream, early_w);
   const int abe = block_elems(act_type_for(type));
   // Two rows at a time through the register-resident kernel beats sixteen at a time through the generic
   // one when the matrix fits in L2 (every pass after the first streams from there).
@@ -755,9 +718,10 @@ int32_t decode_chunked(int type, int64_t m_total, int64_t n, int64_t k, const vo
   for (int64_t m0 = 0; m0 < m_total; m0 += step) {
     const int64_t mc = m_total - m0 < step ? m_total - m0 : step;
     ActPlanes a;
+    a.rec = nullptr;
     a.qs = all.qs + m0 * k;
     a.d = all.d + m0 * (k / abe);
-    a.bsums = all.bsums ? all.bsums + m0 * (k / 16) : nullptr;
+    a.bsums = all.bsums ? all.bsums + (abe == QK_K ? m0 * (k / 256) * kSumStride : m0 * (k / 16)) : nullptr;
     const int32_t st = decode_impl(type, mc, n, k, w, a, y + m0 * n, stream, early_w);
     if (st != kOk) return st;
   }
@@ -1110,9 +1074,7 @@ int32_t fuelq_set_option(int32_t key, int64_t value) {
     case 105: g_opt.dbg_depth = value; return kOk;
     case 106: g_opt.dbg_pre = value; return kOk;
     case 107: g_opt.moe_kernel = value; return kOk;
-    case 111: g_opt.dbg_mb_groups = value; return kOk;
-    case 112: g_opt.dbg_mb_min_m = value; return kOk;
-    case 113: g_opt.dbg_mb_rpc = value; return kOk;
+    case 111: g_opt.dbg_ib_waves = value; return kOk;
     case 114: g_opt.dbg_host_wb = value; return kOk;
     case 115: g_opt.dbg_host_early = value; return kOk;
     case 116: g_opt.dbg_slab_kb = value > 0 ? value : 0; return kOk;
@@ -1253,9 +1215,10 @@ static int32_t qmatmul_integer(int32_t ggml_type, int64_t m_total, int64_t n, in
     st = decode_regs_impl(ggml_type, m_total, n, k, w, none, y, (cudaStream_t)stream, nullptr, x);
     if (st != kNotSupported) return st;
   }
-  st = quantize_act_impl(ggml_type, m_total, k, x, nullptr, workspace, (cudaStream_t)stream);
+  const bool planes = integer_kernel_forced();
+  st = quantize_act_impl(ggml_type, m_total, k, x, nullptr, workspace, (cudaStream_t)stream, planes);
   if (st != kOk) return st;
-  return decode_chunked(ggml_type, m_total, n, k, w, workspace, y, (cudaStream_t)stream, true);
+  return decode_chunked(ggml_type, m_total, n, k, w, workspace, y, (cudaStream_t)stream, true, planes);
 }
 
 int32_t fuelq_qmatmul_sharded(int32_t ggml_type, int64_t m_total, int64_t n_local, int64_t k, const void* w_local,
@@ -1312,7 +1275,7 @@ int32_t fuelq_qmatmul_host(int32_t ggml_type, int64_t m_total, int64_t n, int64_
       if (g_opt.l2_prefetch)
         s1 = prefetch_impl(w, n * (k / block_elems(ggml_type)) * block_bytes(ggml_type), stream);
       unsigned* done = (unsigned*)x_dev;  // the staging area for x is free on this path: its first word counts thread blocks
-      if (s1 == kOk) s1 = quantize_act_impl(ggml_type, m_total, k, xm, nullptr, p, stream, done, g_opt.dbg_host_early != 0);
+      if (s1 == kOk) s1 = quantize_act_impl(ggml_type, m_total, k, xm, nullptr, p, stream, integer_kernel_forced(), done, g_opt.dbg_host_early != 0);
       if (s1 != kOk) return s1;
       // One row in plain launches: the mat-vec kernel's last thread block writes y to the host buffer itself (one launch
       // fewer). With programmatic dependent launch the separate write-back kernel measured faster: it is resident
@@ -1322,7 +1285,7 @@ int32_t fuelq_qmatmul_host(int32_t ggml_type, int64_t m_total, int64_t n, int64_
         s1 = decode_regs_impl(ggml_type, 1, n, k, w, act_planes(p, ggml_type, 1, k), y_dev, stream, nullptr, nullptr, ym, done, true);
         if (s1 != kNotSupported) return s1;
       }
-      s1 = decode_chunked(ggml_type, m_total, n, k, w, p, y_dev, stream, true);
+      s1 = decode_chunked(ggml_type, m_total, n, k, w, p, y_dev, stream, true, integer_kernel_forced());
       if (s1 != kOk) return s1;
       const long long words = (long long)m_total * n;
       const unsigned grid = (unsigned)std::min<long long>((words / 4 + 255) / 256 + 1, 16);
@@ -1607,10 +1570,9 @@ int32_t fuelq_moe_quantize_rows(const float* x, int64_t k, const int32_t* row_id
   if (!x || !row_ids || !packed) return kInvalidProblem;
   if (packed_bytes < act_packed_bytes(kQ4K, n_rows, k)) return kWorkspace;
   if (!aligned(x, 16) || !aligned(packed, 16)) return kMisaligned;
-  const ActPlanes a = act_planes(packed, kQ4K, n_rows, k);
   const int64_t nb = n_rows * (k / 256);
   const cudaError_t e = launch(moe_gather_quantize_kernel, dim3((unsigned)((nb + 7) / 8)), dim3(256), 0, (cudaStream_t)stream, x,
-                               (int)k, (const int*)row_ids, (int)divisor, nb, (int8_t*)a.qs, (float*)a.d, (int16_t*)a.bsums);
+                               (int)k, (const int*)row_ids, (int)divisor, nb, n_rows, act_layout(packed, kQ4K, n_rows, k));
   return e == cudaSuccess ? kOk : kLaunchFailure;
 }
 
@@ -1621,10 +1583,9 @@ int32_t fuelq_moe_swiglu_quantize(const float* gate_up, int64_t f, int64_t n_row
   if (!gate_up || !packed) return kInvalidProblem;
   if (packed_bytes < act_packed_bytes(kQ4K, n_rows, f)) return kWorkspace;
   if (!aligned(gate_up, 16) || !aligned(packed, 16)) return kMisaligned;
-  const ActPlanes a = act_planes(packed, kQ4K, n_rows, f);
   const int64_t nb = n_rows * (f / 256);
   const cudaError_t e = launch(moe_swiglu_quantize_kernel, dim3((unsigned)((nb + 7) / 8)), dim3(256), 0, (cudaStream_t)stream,
-                               gate_up, (int)f, nb, (int8_t*)a.qs, (float*)a.d, (int16_t*)a.bsums);
+                               gate_up, (int)f, nb, n_rows, act_layout(packed, kQ4K, n_rows, f));
   return e == cudaSuccess ? kOk : kLaunchFailure;
 }
 
@@ -1657,14 +1618,9 @@ int32_t fuelq_moe_qmatmul(int32_t ggml_type, int32_t n_experts, int64_t n, int64
   if (n_rows == 0) return kOk;
   if (!w || !packed_act || !expert_offsets || !y) return kInvalidProblem;
   if (!aligned(w, 16) || !aligned(packed_act, 16)) return kMisaligned;
-  if ((g_opt.moe_kernel == 0 && ggml_type != kQ4K) || g_opt.moe_kernel == 3) {
-    const int32_t sm = mma_batch_impl(ggml_type, n_experts, n, k, w, act_planes(const_cast<void*>(packed_act), ggml_type, n_rows, k),
-                                      (const int*)expert_offsets, 0, (const int*)out_rows, y, true, (cudaStream_t)stream);
-    if (sm != kNotSupported) return sm;
-  }
-  if (ggml_type == kQ4K && (g_opt.moe_kernel == 0 || g_opt.moe_kernel == 2)) {
-    const int32_t sm = moe_mma_impl(n_experts, n, k, w, act_planes(const_cast<void*>(packed_act), ggml_type, n_rows, k),
-                                    (const int*)expert_offsets, 0, (const int*)out_rows, y, (cudaStream_t)stream);
+  if (g_opt.moe_kernel == 0) {
+    const int32_t sm = ibatch_impl(ggml_type, n_experts, n, k, w, act_layout(const_cast<void*>(packed_act), ggml_type, n_rows, k),
+                                   (const int*)expert_offsets, n_rows, (const int*)out_rows, y, (cudaStream_t)stream, false);
     if (sm != kNotSupported) return sm;
   }
   DeviceInfo* di;
@@ -1673,9 +1629,10 @@ int32_t fuelq_moe_qmatmul(int32_t ggml_type, int32_t n_experts, int64_t n, int64
   p.row_bytes = (int)(k / 256 * block_bytes(ggml_type));
   if (p.row_bytes % 16) return kNotSupported;  // rows are bulk-copied whole: Q6_K needs k a multiple of 2048
   p.w = (const uint8_t*)w;
-  p.act = act_planes(const_cast<void*>(packed_act), ggml_type, n_rows, k);
+  p.act = act_layout(const_cast<void*>(packed_act), ggml_type, n_rows, k);
   p.offsets = (const int*)expert_offsets;
   p.out_rows = (const int*)out_rows;
+  p.n_rows = n_rows;
   p.y = y;
   p.n = (int)n;
   p.k = (int)k;
@@ -1683,7 +1640,7 @@ int32_t fuelq_moe_qmatmul(int32_t ggml_type, int32_t n_experts, int64_t n, int64
   p.units_per_row = (int)(k / 256) * (ggml_type == kQ4K ? Q4KDecode::kUnitsPerBlock : Q6KDecode::kUnitsPerBlock);
   const size_t header = align_up(sizeof(MoeSmemHeader), 128);
   // shared memory per thread block (two per SM): activation rows of one pass, then the ring of weight stages
-  int act_rows = (int)((40 * 1024) / (k + k / 8 + k / 64 + 64)) / kMoeMT * kMoeMT;
+  int act_rows = (int)((44 * 1024) / (k + k / 4 + k / 64 + 64)) / kMoeMT * kMoeMT;
   if (act_rows > 32) act_rows = 32;
   if (act_rows < kMoeMT) return kNotSupported;
   const size_t act_bytes = align_up(act_packed_bytes(kQ4K, act_rows, k), 128);

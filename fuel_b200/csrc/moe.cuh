@@ -203,10 +203,18 @@ __global__ void __launch_bounds__(1024) moe_bucket_chunks_kernel(const int* topk
   }
 }
 
+// a block of row `row` of n_rows rows, into whichever layout rows of that count have
+__device__ __forceinline__ void moe_store_block(const float (&e)[8], int lane, int64_t row, int b, int64_t blk, int64_t n_rows, const ActPlanes& out) {
+  const Q8KLaneBlock q = q8k_block_quantize(e, lane);
+  if (out.rec)
+    q8k_record_store(q, lane, const_cast<uint8_t*>(out.rec) + (b * n_rows + row) * kActRecord);
+  else
+    q8k_block_store(q, lane, blk, const_cast<int8_t*>(out.qs), const_cast<float*>(out.d), const_cast<int16_t*>(out.bsums));
+}
+
 // ---- gather + Q8_K quantization: sorted row i <- x[row_ids[i] / divisor] (k a multiple of 256)
 __global__ void __launch_bounds__(256) moe_gather_quantize_kernel(const float* x, int k, const int* row_ids, int divisor,
-                                                                  int64_t n_blocks, int8_t* out_qs, float* out_d,
-                                                                  int16_t* out_bsums) {
+                                                                  int64_t n_blocks, int64_t n_rows, ActPlanes out) {
   pdl_launch_dependents();
   pdl_wait();
   const int lane = threadIdx.x & 31;
@@ -219,12 +227,11 @@ __global__ void __launch_bounds__(256) moe_gather_quantize_kernel(const float* x
   const float4* src = reinterpret_cast<const float4*>(x + (size_t)src_row * k + b * 256);
   const float4 v0 = src[lane], v1 = src[32 + lane];
   const float e[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
-  q8k_block_from_regs(e, lane, blk, out_qs, out_d, out_bsums);
+  moe_store_block(e, lane, row, b, blk, n_rows, out);
 }
 
 // ---- silu(gate) * up over rows [gate | up] of width 2f (f a multiple of 256), quantized to Q8_K
-__global__ void __launch_bounds__(256) moe_swiglu_quantize_kernel(const float* gu, int f, int64_t n_blocks, int8_t* out_qs,
-                                                                  float* out_d, int16_t* out_bsums) {
+__global__ void __launch_bounds__(256) moe_swiglu_quantize_kernel(const float* gu, int f, int64_t n_blocks, int64_t n_rows, ActPlanes out) {
   pdl_launch_dependents();
   pdl_wait();
   const int lane = threadIdx.x & 31;
@@ -241,7 +248,7 @@ __global__ void __launch_bounds__(256) moe_swiglu_quantize_kernel(const float* g
   float e[8];
 #pragma unroll
   for (int i = 0; i < 8; ++i) e[i] = (g[i] / (1.0f + expf(-g[i]))) * u[i];
-  q8k_block_from_regs(e, lane, blk, out_qs, out_d, out_bsums);
+  moe_store_block(e, lane, row, b, blk, n_rows, out);
 }
 
 // ---- grouped mat-vec: y[out_row(i), :] = W[e] . act[i] for the sorted rows i of every expert e
@@ -253,6 +260,7 @@ struct MoeParams {
   float* y;              // [rows][n]
   int64_t expert_bytes;  // n * row_bytes
   int n, k, row_bytes, units_per_row, rows_per_stage, num_stages, stage_stride;
+  int64_t n_rows;        // all sorted rows
   int act_rows;          // activation rows held in shared memory per pass over the weights
   int act_smem_off;      // where they live
 };
@@ -329,13 +337,22 @@ __global__ void __launch_bounds__(kDecodeThreads, 2) moe_decode_kernel(const Moe
   // ---------------- consumers
   const ActPlanes sp = act_planes(smem_raw + p.act_smem_off, kQ4K, p.act_rows, p.k);
   const int t = threadIdx.x, nt = 32 * kDecodeConsumerWarps;
-  const int dpr = p.k >> 8, bpr = p.k >> 4;  // block scales / 16-sums per row
+  const int dpr = p.k >> 8, bpr = dpr * kSumStride;  // block scales / int16 units of the sums plane per row
   int g = 0;
   for (int pass = 0; pass < n_pass; ++pass) {
     const int a0 = m_begin + pass * p.act_rows;
     const int ac = (m_count - pass * p.act_rows < p.act_rows) ? m_count - pass * p.act_rows : p.act_rows;
     if (pass > 0) asm volatile("bar.sync 1, %0;" ::"n"(32 * kDecodeConsumerWarps) : "memory");  // previous rows are done with
-    {
+    if (p.act.rec) {  // records back into planes; the f16 sums are whole numbers
+      for (int i = t; i < ac * dpr; i += nt) {
+        const int r = i / dpr, b = i - r * dpr;
+        const uint8_t* rec = p.act.rec + ((size_t)b * p.n_rows + a0 + r) * kActRecord;
+        for (int j = 0; j < 16; ++j) reinterpret_cast<uint4*>(const_cast<int8_t*>(sp.qs) + (size_t)r * p.k + b * 256)[j] = reinterpret_cast<const uint4*>(rec)[j];
+        const_cast<float*>(sp.d)[(size_t)r * dpr + b] = *reinterpret_cast<const float*>(rec + kActRecD);
+        int16_t* bs = const_cast<int16_t*>(sp.bsums) + ((size_t)r * dpr + b) * kSumStride;
+        for (int j = 0; j < 16; ++j) bs[j] = (int16_t)__half2int_rn(reinterpret_cast<const __half*>(rec + kActRecAux)[j]);
+      }
+    } else {
       const uint4* src = reinterpret_cast<const uint4*>(p.act.qs + (size_t)a0 * p.k);
       uint4* dst = reinterpret_cast<uint4*>(const_cast<int8_t*>(sp.qs));
       for (int i = t; i < ac * (p.k >> 4); i += nt) dst[i] = src[i];

@@ -81,6 +81,13 @@ __device__ __forceinline__ Q8KLaneBlock q8k_block_quantize(const float (&e)[8], 
   return b;
 }
 
+// sums of 16-element groups g and 8 + g, in both forms of the plane
+__device__ __forceinline__ void store_sums(int16_t* out, int g, int s0, int s1) {
+  out[g] = (int16_t)s0, out[8 + g] = (int16_t)s1;
+  __half* h = reinterpret_cast<__half*>(out + 16);
+  h[g] = __int2half_rn(s0), h[8 + g] = __int2half_rn(s1);
+}
+
 __device__ __forceinline__ void q8k_block_store(const Q8KLaneBlock& b, int lane, int64_t blk, int8_t* out_qs,
                                                 float* out_d, int16_t* out_bsums) {
   uint32_t* qs = reinterpret_cast<uint32_t*>(out_qs + blk * QK_K);
@@ -88,8 +95,19 @@ __device__ __forceinline__ void q8k_block_store(const Q8KLaneBlock& b, int lane,
   qs[32 + lane] = b.p1;
   if (lane == 0) out_d[blk] = b.d;
   if ((lane & 3) == 0) {
-    out_bsums[blk * 16 + (lane >> 2)] = (int16_t)b.s0;
-    out_bsums[blk * 16 + 8 + (lane >> 2)] = (int16_t)b.s1;
+    store_sums(out_bsums + blk * kSumStride, lane >> 2, b.s0, b.s1);
+  }
+}
+
+// the same block as a record
+__device__ __forceinline__ void q8k_record_store(const Q8KLaneBlock& b, int lane, uint8_t* rec) {
+  uint32_t* qs = reinterpret_cast<uint32_t*>(rec);
+  qs[lane] = b.p0;
+  qs[32 + lane] = b.p1;
+  if (lane == 0) *reinterpret_cast<float*>(rec + kActRecD) = b.d;
+  if ((lane & 3) == 0) {
+    __half* h = reinterpret_cast<__half*>(rec + kActRecAux);
+    h[lane >> 2] = __int2half_rn(b.s0), h[8 + (lane >> 2)] = __int2half_rn(b.s1);
   }
 }
 
@@ -101,7 +119,8 @@ __device__ __forceinline__ void q8k_block_from_regs(const float (&e)[8], int lan
 template <bool kRefLayout>
 __global__ void __launch_bounds__(256) quantize_q8k_kernel(const float* x, int64_t n_blocks,
                                                            uint8_t* out_ref, int8_t* out_qs,
-                                                           float* out_d, int16_t* out_bsums, unsigned* zero_word,
+                                                           float* out_d, int16_t* out_bsums, uint8_t* out_rec, int rows, int nblk,
+                                                           unsigned* zero_word,
                                                            int early_x, int late_trigger) {
   // early_x: x does not come from an earlier kernel of the stream (host data, final when the call was made), so it is
   // loaded before the wait for the predecessors and only the stores are ordered after them: a slow read (host memory
@@ -124,77 +143,23 @@ __global__ void __launch_bounds__(256) quantize_q8k_kernel(const float* x, int64
   }
   if (zero_word && blockIdx.x == 0 && threadIdx.x == 0) *zero_word = 0u;  // a counter the next kernel starts from
 
-  // first-max-wins scan, in index order within the lane
-  float amax = 0.f, smax = 0.f;
-  int idx = 0;
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const float a = fabsf(e[i]);
-    if (amax < a) {
-      amax = a;
-      smax = e[i];
-      idx = (i < 4 ? 4 * lane + i : 128 + 4 * lane + (i - 4));
-    }
-  }
-#pragma unroll
-  for (int off = 16; off > 0; off >>= 1) {
-    const float oa = __shfl_xor_sync(0xffffffffu, amax, off);
-    const float os = __shfl_xor_sync(0xffffffffu, smax, off);
-    const int oi = __shfl_xor_sync(0xffffffffu, idx, off);
-    if (oa > amax || (oa == amax && oi < idx)) {
-      amax = oa;
-      smax = os;
-      idx = oi;
-    }
-  }
-
-  int q[8];
-  float d;
-  if (amax == 0.f) {
-    d = 0.f;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) q[i] = 0;
-  } else {
-    const float iscale = -128.0f / smax;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const float r = fminf(roundf(iscale * e[i]), 127.0f);
-      q[i] = max(__float2int_rz(r), -128);
-    }
-    d = 1.0f / iscale;
-  }
-  // sums of 16 consecutive values = 4 neighbouring lanes x 4 values
-  int s0 = q[0] + q[1] + q[2] + q[3];
-  int s1 = q[4] + q[5] + q[6] + q[7];
-  s0 += __shfl_xor_sync(0xffffffffu, s0, 1);
-  s1 += __shfl_xor_sync(0xffffffffu, s1, 1);
-  s0 += __shfl_xor_sync(0xffffffffu, s0, 2);
-  s1 += __shfl_xor_sync(0xffffffffu, s1, 2);
-
-  const uint32_t p0 = (uint32_t)(q[0] & 0xff) | ((uint32_t)(q[1] & 0xff) << 8) | ((uint32_t)(q[2] & 0xff) << 16) |
-                      ((uint32_t)(q[3] & 0xff) << 24);
-  const uint32_t p1 = (uint32_t)(q[4] & 0xff) | ((uint32_t)(q[5] & 0xff) << 8) | ((uint32_t)(q[6] & 0xff) << 16) |
-                      ((uint32_t)(q[7] & 0xff) << 24);
+  const Q8KLaneBlock q = q8k_block_quantize(e, lane);
   if (kRefLayout) {
     uint8_t* b = out_ref + blk * Q8KL::kBytes;  // 292-byte blocks are 4-byte aligned
-    if (lane == 0) *reinterpret_cast<float*>(b + Q8KL::kOffD) = d;
+    if (lane == 0) *reinterpret_cast<float*>(b + Q8KL::kOffD) = q.d;
     uint32_t* qs = reinterpret_cast<uint32_t*>(b + Q8KL::kOffQs);
-    qs[lane] = p0;
-    qs[32 + lane] = p1;
+    qs[lane] = q.p0;
+    qs[32 + lane] = q.p1;
     int16_t* bs = reinterpret_cast<int16_t*>(b + Q8KL::kOffBsums);
     if ((lane & 3) == 0) {
-      bs[lane >> 2] = (int16_t)s0;
-      bs[8 + (lane >> 2)] = (int16_t)s1;
+      bs[lane >> 2] = (int16_t)q.s0;
+      bs[8 + (lane >> 2)] = (int16_t)q.s1;
     }
+  } else if (out_rec) {
+    const int64_t row = blk / nblk;
+    q8k_record_store(q, lane, out_rec + ((blk - row * nblk) * rows + row) * kActRecord);
   } else {
-    uint32_t* qs = reinterpret_cast<uint32_t*>(out_qs + blk * QK_K);
-    qs[lane] = p0;
-    qs[32 + lane] = p1;
-    if (lane == 0) out_d[blk] = d;
-    if ((lane & 3) == 0) {
-      out_bsums[blk * 16 + (lane >> 2)] = (int16_t)s0;
-      out_bsums[blk * 16 + 8 + (lane >> 2)] = (int16_t)s1;
-    }
+    q8k_block_store(q, lane, blk, out_qs, out_d, out_bsums);
   }
 }
 
@@ -205,7 +170,7 @@ __global__ void __launch_bounds__(256) quantize_q8k_kernel(const float* x, int64
 template <bool kRefLayout, bool kQ81 = false>
 __global__ void __launch_bounds__(256) quantize_q8_0_kernel(const float* x, int64_t n_groups /* of 256 */,
                                                             int64_t n_blocks32, uint8_t* out_ref,
-                                                            int8_t* out_qs, float* out_d, unsigned* zero_word,
+                                                            int8_t* out_qs, float* out_d, uint8_t* out_rec, int rows, int nblk, unsigned* zero_word,
                                                             int early_x, int late_trigger, float* out_s = nullptr) {
   if (!late_trigger) pdl_launch_dependents();
   if (!early_x) pdl_wait();
@@ -271,6 +236,12 @@ __global__ void __launch_bounds__(256) quantize_q8_0_kernel(const float* x, int6
         if (sub == 0) b[0] = (uint32_t)__half_as_ushort(h1) | ((uint32_t)__half_as_ushort(sh1) << 16);
         b[1 + sub] = p1;
       }
+    } else if (out_rec) {
+      const int64_t row = grp / nblk;
+      uint8_t* rec = out_rec + ((grp - row * nblk) * rows + row) * kActRecordMin;
+      reinterpret_cast<uint32_t*>(rec)[lane] = p0, reinterpret_cast<uint32_t*>(rec)[32 + lane] = p1;
+      float* aux = reinterpret_cast<float*>(rec + kActRecAux) + (lane >> 3);
+      if (sub == 0) aux[0] = __half2float(h0), aux[4] = __half2float(h1), aux[8] = __half2float(sh0), aux[12] = __half2float(sh1);
     } else {
       uint32_t* qs = reinterpret_cast<uint32_t*>(out_qs + base);
       if (ok0) {
@@ -298,6 +269,12 @@ __global__ void __launch_bounds__(256) quantize_q8_0_kernel(const float* x, int6
       b[1 + 2 * sub] = (uint16_t)(p1 & 0xffff);
       b[2 + 2 * sub] = (uint16_t)(p1 >> 16);
     }
+  } else if (out_rec) {
+    const int64_t row = grp / nblk;
+    uint8_t* rec = out_rec + ((grp - row * nblk) * rows + row) * kActRecord;
+    reinterpret_cast<uint32_t*>(rec)[lane] = p0, reinterpret_cast<uint32_t*>(rec)[32 + lane] = p1;
+    float* aux = reinterpret_cast<float*>(rec + kActRecAux) + (lane >> 3);
+    if (sub == 0) aux[0] = __half2float(h0), aux[4] = __half2float(h1);
   } else {
     uint32_t* qs = reinterpret_cast<uint32_t*>(out_qs + base);
     if (ok0) {
