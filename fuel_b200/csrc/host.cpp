@@ -224,9 +224,16 @@ std::shared_ptr<SharedWorkspace> SharedWorkspace::of(const Device& dev) {
   if (!ws) slot = ws = std::make_shared<SharedWorkspace>();
   return ws;
 }
-void* SharedWorkspace::ensure(const Device& dev, size_t need) {
-  if (bytes() < need || buffers.empty())
-    buffers.emplace_back(dev, std::max<size_t>({need, 2 * bytes(), (size_t)1 << 20}), false);
+void* SharedWorkspace::ensure(const Device& dev, size_t need, size_t least) {
+  if (bytes() < need || buffers.empty()) {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;  // an allocation is no part of a capture under way
+    cuda_check(cudaThreadExchangeStreamCaptureMode(&mode), "cudaThreadExchangeStreamCaptureMode");
+    struct Restore {
+      cudaStreamCaptureMode* mode;
+      ~Restore() { cudaThreadExchangeStreamCaptureMode(mode); }
+    } restore{&mode};
+    buffers.emplace_back(dev, std::max({need, 2 * bytes(), least}), false);
+  }
   return buffers.back().ptr();
 }
 
@@ -238,12 +245,20 @@ void QStorage::fwd_into(const Shape& self_shape, const float* x, const Shape& in
   fwd_rows(n, k, x, elem_count(in_shape) / (k ? k : 1), y);
 }
 
+// The legacy default stream can't be captured, so the usual caller is spared the query.
+static bool capturing(const Device& dev) {
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  return dev.stream() && cs(dev) != cudaStreamLegacy && cudaStreamIsCapturing(cs(dev), &status) == cudaSuccess &&
+         status == cudaStreamCaptureStatusActive;
+}
+
 void QStorage::fwd_rows(int64_t n, int64_t k, const float* x, int64_t m, float* y) const {
   dev_.make_current();
   const size_t need = fuelq_qmatmul_workspace_bytes((int32_t)dtype_, m, n, k);
-  SharedWorkspace& ws = *workspace_;
+  const bool recorded = capturing(dev_);
+  SharedWorkspace& ws = recorded ? *captured_ : *workspace_;
   std::lock_guard<std::mutex> lock(ws.mutex);
-  void* scratch = ws.ensure(dev_, need);
+  void* scratch = ws.ensure(dev_, need, recorded ? 16 : (size_t)1 << 20);
   check(fuelq_qmatmul((int32_t)dtype_, m, n, k, buf_.ptr(), x, y, scratch, ws.bytes(), dev_.stream()), "fuelq_qmatmul");
 }
 

@@ -78,7 +78,7 @@ class DeviceBuffer {
   int ordinal_ = 0;
 };
 
-// Device scratch for fwd, shared by every storage on one (device, stream): the calls of a stream run in order, so one buffer
+// Device scratch for fwd, shared by every storage on one (device, stream), calls under stream capture aside: the calls of a stream run in order, so one buffer
 // serves all of a model's linears (one each would cost a model of two hundred of them gigabytes, and an allocation with a
 // device synchronization on each one's first call). Growing keeps the smaller buffers, since kernels in flight or captured
 // graphs may hold their addresses; growth is at least twofold, so the total stays below twice the largest need, and all of
@@ -88,7 +88,7 @@ struct SharedWorkspace {
   std::mutex mutex;
   std::vector<DeviceBuffer> buffers;  // the last one is the largest
   static std::shared_ptr<SharedWorkspace> of(const Device& dev);
-  void* ensure(const Device& dev, size_t bytes);  // with `mutex` held
+  void* ensure(const Device& dev, size_t bytes, size_t least);  // with `mutex` held; at least `least` when it allocates
   size_t bytes() const { return buffers.empty() ? 0 : buffers.back().bytes(); }
 };
 
@@ -135,6 +135,9 @@ class QStorage {
   size_t len_ = 0;
   DeviceBuffer buf_;
   std::shared_ptr<SharedWorkspace> workspace_;
+  // Calls recorded into a graph get scratch of this storage alone: the graph may be replayed on another stream, beside the
+  // calls that share workspace_.
+  std::unique_ptr<SharedWorkspace> captured_ = std::make_unique<SharedWorkspace>();
 };
 
 class QTensor {
