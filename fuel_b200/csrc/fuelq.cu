@@ -679,6 +679,7 @@ int32_t ibatch_fmt(int n_groups, int64_t n, int64_t k, const void* w, const ActP
 int32_t ibatch_impl(int type, int n_groups, int64_t n, int64_t k, const void* w, const ActPlanes& act, const int* offsets,
                     int64_t n_rows, const int* out_rows, float* y, cudaStream_t stream, bool early_w) {
   if (k % 256 || n > INT32_MAX - 64 || n_groups > 65535 || n_rows > (1 << 28)) return kNotSupported;
+  if (!act.rec && n_rows > 1) return kNotSupported;  // planes are read for single rows only
 #define FQ_IB(T, F) \
   case T: return ibatch_fmt<F>(n_groups, n, k, w, act, offsets, n_rows, out_rows, y, stream, early_w)
   switch (type) {
@@ -1274,8 +1275,11 @@ int32_t fuelq_qmatmul_host(int32_t ggml_type, int64_t m_total, int64_t n, int64_
       int32_t s1 = kOk;
       if (g_opt.l2_prefetch)
         s1 = prefetch_impl(w, n * (k / block_elems(ggml_type)) * block_bytes(ggml_type), stream);
+      // Reading x beside the stream's earlier kernels needs the promise of FUELQ_OPT_PDL: one of them may be the write-back
+      // of a call whose result is this call's x.
+      const bool early_x = g_opt.pdl && g_opt.dbg_host_early;
       unsigned* done = (unsigned*)x_dev;  // the staging area for x is free on this path: its first word counts thread blocks
-      if (s1 == kOk) s1 = quantize_act_impl(ggml_type, m_total, k, xm, nullptr, p, stream, integer_kernel_forced(), done, g_opt.dbg_host_early != 0);
+      if (s1 == kOk) s1 = quantize_act_impl(ggml_type, m_total, k, xm, nullptr, p, stream, integer_kernel_forced(), done, early_x);
       if (s1 != kOk) return s1;
       // One row in plain launches: the mat-vec kernel's last thread block writes y to the host buffer itself (one launch
       // fewer). With programmatic dependent launch the separate write-back kernel measured faster: it is resident
@@ -1308,7 +1312,7 @@ int32_t fuelq_qmatmul_host(int32_t ggml_type, int64_t m_total, int64_t n, int64_
 // device pointers but no allocator, or a process whose memory pool is owned by another runtime.
 // For them the activation scratch lives in the library image itself: a fixed device array that
 // every GPU loading the library carries until the process exits.
-constexpr size_t kStaticScratchBytes = 1u << 20;  // 1 MiB: e.g. m_total * k up to ~900k elements
+constexpr size_t kStaticScratchBytes = 5u << 18;  // 1.25 MiB: m_total * k up to a million elements
 static __device__ __align__(256) unsigned char g_static_scratch[kStaticScratchBytes];
 
 size_t fuelq_static_scratch_bytes(void) { return kStaticScratchBytes; }
