@@ -38,7 +38,6 @@ struct Options {
   int64_t prefill_tf32 = 0;   // tensor-core path in tf32 instead of 16-bit operands
   int64_t prefill_bf16 = 0;   // 16-bit operands as bf16 instead of f16
   int64_t fused_quant = 0;    // f32 activations with m <= 2: quantize inside the mat-vec kernel
-  int64_t dbg_ib_waves = 0;    // grouped matmul: thread blocks per SM in all
   int64_t dbg_host_wb = 0;     // write-back to a host buffer: 0 = by launch mode, 1 = own kernel, 2 = inside the mat-vec kernel
   int64_t dbg_host_early = 1;  // host activations loaded before the wait for earlier kernels
   int64_t dbg_slab_kb = 0;     // tensor-core path through dequantized slabs: slab size in KiB (0 = 128 MiB)
@@ -566,10 +565,10 @@ int32_t prefetch_impl(const void* w, int64_t bytes, cudaStream_t stream) {
 }
 
 // ---- a few to a few dozen rows on the integer tensor cores (ibatch.cuh): every format, k a multiple of 256
-template <class F, int MT>
+template <class F, int MT, bool kGrouped>
 cudaError_t launch_ibatch(const IbParams& p, dim3 grid, int warps, size_t smem, cudaStream_t stream) {
   static bool attr_set[64] = {};
-  auto kern = ibatch_kernel<F, MT>;
+  auto kern = ibatch_kernel<F, MT, kGrouped>;
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
@@ -621,7 +620,7 @@ bool plan_ibatch(IbParams* p, int tiles, int warps, size_t budget, size_t* smem)
   return false;
 }
 
-template <class F>
+template <class F, bool kGrouped>
 int32_t ibatch_fmt(int n_groups, int64_t n, int64_t k, const void* w, const ActPlanes& act, const int* offsets, int64_t n_rows,
                    const int* out_rows, float* y, cudaStream_t stream, bool early_w) {
   DeviceInfo* di;
@@ -640,38 +639,40 @@ int32_t ibatch_fmt(int n_groups, int64_t n, int64_t k, const void* w, const ActP
   p.row_bytes = p.nblk * F::kBytes256;
   p.group_bytes = n * (int64_t)p.row_bytes;
   p.total_bytes = (int64_t)n_groups * p.group_bytes;
-  const int n_tiles = (int)((n + 15) / 16);
-  int warps = kIbMaxWarps, per_group;
-  size_t budget = (size_t)di->max_smem_optin, smem = 0;
-  if (!offsets) {
+  p.n_groups = n_groups;
+  const int64_t n_tiles = (n + 15) / 16;
+  int warps = kIbMaxWarps;
+  size_t smem = 0;
+  int64_t blocks = g_opt.decode_grid > 0 ? g_opt.decode_grid : di->sm_count;
+  if constexpr (!kGrouped) {
     p.rows_cap = n_rows >= kIbMaxRows ? kIbMaxRows : (int)((n_rows + 7) & ~7ll);
-    per_group = di->sm_count;
     if (p.rows_cap > 32) warps = kIbMaxWarps / 2;  // twice the registers a thread
+    if (blocks > n_tiles) blocks = n_tiles;
+    if (!plan_ibatch<F>(&p, (int)((n_tiles + blocks - 1) / blocks), warps, (size_t)di->max_smem_optin, &smem)) return kNotSupported;
   } else {
-    // Routed rows: enough rows per pass for most groups (their mean and twice its root), two thread blocks of eight warps
-    // per SM, so that one computes while the other stages; several blocks per group, as few groups may have rows.
+    // Routed rows: enough rows per pass for most groups (their mean and twice its root), and two thread blocks of eight warps
+    // per SM, so that one computes while the other stages. The kernel deals the tiles of the groups that have rows out
+    // evenly; a grid per group left the SMs to wait for the largest groups, and for blocks of groups without rows.
     const double mean = (double)n_rows / n_groups;
     int cap = ((int)(mean + 2.0 * sqrt(mean)) + 8) & ~7;
     p.rows_cap = cap < 8 ? 8 : cap > kIbMaxRows ? kIbMaxRows : cap;
     warps = kIbMaxWarps / 2;
-    budget = ((size_t)di->max_smem_optin + 1024) / 2 - 1024;
-    const int64_t live = n_rows < n_groups ? n_rows : n_groups;
-    per_group = (int)((int64_t)(g_opt.dbg_ib_waves ? g_opt.dbg_ib_waves : 4) * di->sm_count / live) + 1;
+    const int64_t all = n_tiles * (n_rows < n_groups ? n_rows : n_groups);
+    if (g_opt.decode_grid == 0) blocks = 2 * di->sm_count;
+    if (blocks > all) blocks = all;
+    const int64_t each = (all + blocks - 1) / blocks;
+    const int tiles = (int)(each < n_tiles ? each : n_tiles);
+    if (!plan_ibatch<F>(&p, tiles, warps, ((size_t)di->max_smem_optin + 1024) / 2 - 1024, &smem)) {
+      if (g_opt.decode_grid == 0 && blocks > di->sm_count) blocks = di->sm_count;
+      if (!plan_ibatch<F>(&p, tiles, warps, (size_t)di->max_smem_optin, &smem)) return kNotSupported;
+    }
   }
-  if (g_opt.decode_grid > 0) per_group = (int)g_opt.decode_grid;
-  if (per_group > n_tiles) per_group = n_tiles;
-  if (per_group < 1) per_group = 1;
-  const int tiles = (n_tiles + per_group - 1) / per_group;
-  if (!plan_ibatch<F>(&p, tiles, warps, budget, &smem)) {
-    if (!offsets) return kNotSupported;
-    if (!plan_ibatch<F>(&p, tiles, warps, (size_t)di->max_smem_optin, &smem)) return kNotSupported;
-  }
-  const dim3 grid((unsigned)per_group, (unsigned)n_groups);
+  const dim3 grid((unsigned)blocks);
   cudaError_t e;
-  if (p.rows_cap <= 8) e = launch_ibatch<F, 1>(p, grid, warps, smem, stream);
-  else if (p.rows_cap <= 16) e = launch_ibatch<F, 2>(p, grid, warps, smem, stream);
-  else if (p.rows_cap <= 32) e = launch_ibatch<F, 4>(p, grid, warps, smem, stream);
-  else e = launch_ibatch<F, 8>(p, grid, warps, smem, stream);
+  if (p.rows_cap <= 8) e = launch_ibatch<F, 1, kGrouped>(p, grid, warps, smem, stream);
+  else if (p.rows_cap <= 16) e = launch_ibatch<F, 2, kGrouped>(p, grid, warps, smem, stream);
+  else if (p.rows_cap <= 32) e = launch_ibatch<F, 4, kGrouped>(p, grid, warps, smem, stream);
+  else e = launch_ibatch<F, 8, kGrouped>(p, grid, warps, smem, stream);
   return e == cudaSuccess ? kOk : kLaunchFailure;
 }
 
@@ -680,8 +681,13 @@ int32_t ibatch_impl(int type, int n_groups, int64_t n, int64_t k, const void* w,
                     int64_t n_rows, const int* out_rows, float* y, cudaStream_t stream, bool early_w) {
   if (k % 256 || n > INT32_MAX - 64 || n_groups > 65535 || n_rows > (1 << 28)) return kNotSupported;
   if (!act.rec && n_rows > 1) return kNotSupported;  // planes are read for single rows only
+  if (offsets) {
+    if (type == kQ4K) return ibatch_fmt<IbQ4K, true>(n_groups, n, k, w, act, offsets, n_rows, out_rows, y, stream, early_w);
+    if (type == kQ6K) return ibatch_fmt<IbQ6K, true>(n_groups, n, k, w, act, offsets, n_rows, out_rows, y, stream, early_w);
+    return kNotSupported;
+  }
 #define FQ_IB(T, F) \
-  case T: return ibatch_fmt<F>(n_groups, n, k, w, act, offsets, n_rows, out_rows, y, stream, early_w)
+  case T: return ibatch_fmt<F, false>(n_groups, n, k, w, act, offsets, n_rows, out_rows, y, stream, early_w)
   switch (type) {
     FQ_IB(kQ4K, IbQ4K);
     FQ_IB(kQ5K, IbQ5K);
@@ -1075,7 +1081,6 @@ int32_t fuelq_set_option(int32_t key, int64_t value) {
     case 105: g_opt.dbg_depth = value; return kOk;
     case 106: g_opt.dbg_pre = value; return kOk;
     case 107: g_opt.moe_kernel = value; return kOk;
-    case 111: g_opt.dbg_ib_waves = value; return kOk;
     case 114: g_opt.dbg_host_wb = value; return kOk;
     case 115: g_opt.dbg_host_early = value; return kOk;
     case 116: g_opt.dbg_slab_kb = value > 0 ? value : 0; return kOk;

@@ -50,8 +50,8 @@ struct IbParams {
   int64_t total_bytes;   // n_groups * group_bytes
   int fixed_rows;
   int64_t act_rows;      // rows of the records
-  int early_w;           // dense batch: the weights are streamed before the wait for the preceding kernel
-  int n, nblk, row_bytes;
+  int early_w;           // one matrix: the weights are streamed before the wait for the preceding kernel
+  int n, nblk, row_bytes, n_groups;
   int rows_cap;          // activation rows per pass (a multiple of 8, at most 8 * MT)
   int kp;                // shares of k; the warps of a tile
   int share_q, share_rem;  // blocks per share: share_q, one more in the first share_rem
@@ -133,6 +133,11 @@ __device__ __forceinline__ int ib_sbyte(uint32_t w, int i) { return (int)(int8_t
 __device__ __forceinline__ uint32_t ib_h2(int a, int b) {  // two small integers as packed f16
   const __half2 h = __floats2half2_rn((float)a, (float)b);
   return *reinterpret_cast<const uint32_t*>(&h);
+}
+
+// Cost of a tile for a group of r rows, in 8-row tiles: its unpacking and streaming weigh about as much as three of them
+__device__ __forceinline__ int ib_group_cost(int r, int rows_cap) {
+  return r > 0 ? 3 * ((r + rows_cap - 1) / rows_cap) + ((r + 7) >> 3) : 0;
 }
 
 // Where a warp's operands are: shared addresses
@@ -502,18 +507,15 @@ using IbQ4_1 = Ib32<4, true>;
 using IbQ5_1 = Ib32<5, true>;
 
 // ------------------------------------------------------------------------------------------------ kernel
-template <class F, int MT>
-__global__ void __launch_bounds__(32 * (MT > 4 ? kIbMaxWarps / 2 : kIbMaxWarps), 1) ibatch_kernel(const IbParams p) {
+// kGrouped: the rows of many matrices' groups, two blocks of half the warps a SM; else one matrix and one block a SM
+template <class F, int MT, bool kGrouped>
+__global__ void __launch_bounds__(32 * (kGrouped || MT > 4 ? kIbMaxWarps / 2 : kIbMaxWarps), kGrouped && MT <= 4 ? 2 : 1) ibatch_kernel(const IbParams p) {
   extern __shared__ __align__(128) uint8_t smem_raw[];
   uint64_t* full = reinterpret_cast<uint64_t*>(smem_raw);  // [2]: an activation buffer's copies have landed
   const uint32_t smem = smem_u32(smem_raw);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int grp = blockIdx.y;
-  // this block's share of the weight rows, in whole 16-row tiles
   const int n_tiles = (p.n + 15) >> 4;
-  const int t_begin = (int)((int64_t)n_tiles * blockIdx.x / gridDim.x), t_end = (int)((int64_t)n_tiles * (blockIdx.x + 1) / gridDim.x);
-  const int rounds = (t_end - t_begin + p.tg - 1) / p.tg;
-  const bool early = p.early_w && !p.offsets;
+  const bool early = !kGrouped && p.early_w;
   if (threadIdx.x == 0) {
     mbar_init(&full[0], 1);
     mbar_init(&full[1], 1);
@@ -522,13 +524,61 @@ __global__ void __launch_bounds__(32 * (MT > 4 ? kIbMaxWarps / 2 : kIbMaxWarps),
   __syncthreads();
   pdl_launch_dependents();
   if (!early) pdl_wait();
-  const int m_begin = p.offsets ? p.offsets[grp] : 0;
-  const int m_count = p.offsets ? p.offsets[grp + 1] - m_begin : p.fixed_rows;
-  if (m_count <= 0 || rounds <= 0) {  // nothing is streamed for a group without rows
+
+  // This block's share of the work: whole 16-row tiles of one matrix, or of several groups' (a segment each), equal in cost
+  // to every other block's. `base` is the cost before group grp, per tile of every group; lo and hi are in cost * n_tiles.
+  int grp = 0, m_begin = 0, m_count = p.fixed_rows, t_begin, t_end;
+  int base = 0, cost = 0;
+  int64_t lo = 0, hi = 0;
+  if constexpr (!kGrouped) {
+    t_begin = (int)((int64_t)n_tiles * blockIdx.x / gridDim.x), t_end = (int)((int64_t)n_tiles * (blockIdx.x + 1) / gridDim.x);
+  } else {
+    int total = 0;
+    for (int g = lane; g < p.n_groups; g += 32) total += ib_group_cost(p.offsets[g + 1] - p.offsets[g], p.rows_cap);
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) total += __shfl_xor_sync(0xffffffffu, total, off);
+    lo = (int64_t)total * n_tiles * blockIdx.x / gridDim.x, hi = (int64_t)total * n_tiles * (blockIdx.x + 1) / gridDim.x;
+    for (;; grp += 32) {  // the group that lo falls into
+      if (grp >= p.n_groups) return;
+      const int mine = grp + lane < p.n_groups ? ib_group_cost(p.offsets[grp + lane + 1] - p.offsets[grp + lane], p.rows_cap) : 0;
+      int upto = mine;
+#pragma unroll
+      for (int off = 1; off < 32; off <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, upto, off);
+        if (lane >= off) upto += v;
+      }
+      const unsigned past = __ballot_sync(0xffffffffu, (int64_t)(base + upto) * n_tiles > lo);
+      if (past) {
+        const int l = __ffs((int)past) - 1;
+        base += __shfl_sync(0xffffffffu, upto - mine, l);
+        grp += l;
+        break;
+      }
+      base += __shfl_sync(0xffffffffu, upto, 31);
+    }
+  }
+  // the next segment with tiles in it, from group grp on
+  auto segment = [&]() -> bool {
+    if constexpr (!kGrouped) {
+      return t_begin < t_end;
+    } else {
+      for (; grp < p.n_groups && (int64_t)base * n_tiles < hi; ++grp, base += cost) {
+        m_begin = p.offsets[grp], m_count = p.offsets[grp + 1] - m_begin;
+        cost = ib_group_cost(m_count, p.rows_cap);
+        if (cost == 0) continue;
+        const int64_t l = lo - (int64_t)base * n_tiles, h = hi - (int64_t)base * n_tiles;
+        t_begin = l <= 0 ? 0 : (int)((l + cost - 1) / cost);
+        const int64_t e = (h + cost - 1) / cost;
+        t_end = e < n_tiles ? (int)e : n_tiles;
+        if (t_begin < t_end) return true;
+      }
+      return false;
+    }
+  };
+  if (!segment()) {
     pdl_wait();
     return;
   }
-  const int n_pass = (m_count + p.rows_cap - 1) / p.rows_cap;
   const int kpart = warp % p.kp, slot = warp / p.kp;  // warps past kp * tg have no tile but stage activations
   const int b_begin = kpart * p.share_q + (kpart < p.share_rem ? kpart : p.share_rem), b_end = b_begin + p.share_q + (kpart < p.share_rem);
   const bool has_slot = slot < p.tg;
@@ -539,11 +589,17 @@ __global__ void __launch_bounds__(32 * (MT > 4 ? kIbMaxWarps / 2 : kIbMaxWarps),
   // ---- weight stream of this warp: its tiles' blocks, round after round, pass after pass
   const uint32_t stage_bytes = 16u * F::kPitch;
   const uint32_t wst = smem + kIbHeader + (uint32_t)(warp * p.stages) * stage_bytes;
-  const int64_t gbase = (int64_t)grp * p.group_bytes;
-  const int my_rounds = has_slot ? (t_end - t_begin - slot + p.tg - 1) / p.tg : 0;  // tiles slot, slot + tg, ...
   const int nb = b_end - b_begin;
-  const int per_pass = my_rounds * nb, total_steps = per_pass * n_pass;
-  int f_tile = t_begin + slot, f_b = b_begin, f_stage = 0, f_left = total_steps;  // next block to fetch
+  int64_t gbase;
+  int n_pass, rounds;
+  int f_tile, f_b, f_stage = 0, f_left;  // next block to fetch
+  auto start_stream = [&]() {  // for the segment's tiles slot, slot + tg, ...
+    gbase = kGrouped ? (int64_t)grp * p.group_bytes : 0;
+    n_pass = (m_count + p.rows_cap - 1) / p.rows_cap;
+    rounds = (t_end - t_begin + p.tg - 1) / p.tg;
+    const int mine = has_slot && t_end - t_begin > slot ? (t_end - t_begin - slot + p.tg - 1) / p.tg : 0;
+    f_tile = t_begin + slot, f_b = b_begin, f_left = mine * nb * n_pass;
+  };
   constexpr int kPieces = F::kAligned ? F::kBytes256 / 16 : F::kPitch / 16 - 1, kCopies = (16 * kPieces + 31) / 32;
   int rc[kCopies];  // this lane's pieces: row | piece << 8, or -1
 #pragma unroll
@@ -592,14 +648,13 @@ __global__ void __launch_bounds__(32 * (MT > 4 ? kIbMaxWarps / 2 : kIbMaxWarps),
   // ---- activation staging: chunk c of the pass that starts at row a0 into buffer `buf`. Slot s holds the s % bpc-th block of
   // the chunk of share s / bpc: the rows' records, one bulk copy (a lane of warp 0 each). Rows past `ac` keep whatever is
   // there: a row is a column of the MMAs' results, and theirs are not stored.
-  const int rows = n_pass == 1 ? (m_count + 7) & ~7 : p.rows_cap;
   constexpr int kRec = ib_rec(F::kAct);
-  const int slot_bytes = rows * kRec;
+  int slot_bytes, bpc, n_chunks;
   auto stage_acts = [&](int a0, int ac, int c, int buf) {
     const uint32_t base = (uint32_t)(p.act_off + buf * p.act_buf);
-    const int slots = p.kp * p.bpc;
+    const int slots = p.kp * bpc;
     auto slot_block = [&](int s) -> int {  // or -1
-      const int sh = s / p.bpc, b0 = sh * p.share_q + (sh < p.share_rem ? sh : p.share_rem), j = c * p.bpc + s - sh * p.bpc;
+      const int sh = s / bpc, b0 = sh * p.share_q + (sh < p.share_rem ? sh : p.share_rem), j = c * bpc + s - sh * bpc;
       return j < p.share_q + (sh < p.share_rem) ? b0 + j : -1;
     };
     if (p.act.rec) {
@@ -642,116 +697,126 @@ __global__ void __launch_bounds__(32 * (MT > 4 ? kIbMaxWarps / 2 : kIbMaxWarps),
     }
   };
 
-  // prologue: all but one stage of weights (before the wait for the predecessor where allowed), then the first activations
-  if (early) {
-    for (int i = 0; i < p.stages - 1; ++i) fetch();
-    pdl_wait();
-  }
   float* part = reinterpret_cast<float*>(smem_raw + p.part_off);
   int step_stage = 0;
-  for (int pass = 0; pass < n_pass; ++pass) {
-    const int a0 = m_begin + pass * p.rows_cap;
-    const int ac = m_count - pass * p.rows_cap < p.rows_cap ? m_count - pass * p.rows_cap : p.rows_cap;
-    cx.nt = (ac + 7) >> 3;
-    if (pass > 0) __syncthreads();  // the previous pass's activations are done with
-    stage_acts(a0, ac, 0, 0);
-    if (pass == 0 && !early)
-      for (int i = 0; i < p.stages - 1; ++i) fetch();
-    if (!p.act.rec) {
-      ib_wait(pass == 0 && !early ? p.stages - 1 : 0);
-      __syncthreads();
+  for (bool first = true;; first = false) {
+    start_stream();
+    // all but one stage of weights (before the wait for the predecessor where allowed), then the first activations
+    for (int i = 0; i < p.stages - 1; ++i) fetch();
+    if (first && early) pdl_wait();
+    // the plan's chunks are for rows_cap rows: fewer need fewer chunks
+    slot_bytes = (n_pass == 1 ? (m_count + 7) & ~7 : p.rows_cap) * kRec;
+    bpc = p.bpc, n_chunks = p.n_chunks;
+    if (kGrouped && n_chunks > 1) {
+      const int share = p.share_q + (p.share_rem > 0);
+      if (p.kp * share * slot_bytes <= 2 * p.act_buf) bpc = share, n_chunks = 1;
+      else bpc = p.act_buf / (p.kp * slot_bytes), n_chunks = (share + bpc - 1) / bpc;
     }
-    acts_landed(0);
-    int buf = 0;
-    for (int round = 0; round < rounds; ++round) {
-      float facc[MT][4];
-#pragma unroll
-      for (int mt = 0; mt < MT; ++mt)
-#pragma unroll
-        for (int i = 0; i < 4; ++i) facc[mt][i] = 0.f;
-      const int tile = t_begin + round * p.tg + slot;
-      const bool live = has_slot && tile < t_end;
-      for (int c = 0; c < p.n_chunks; ++c) {
-        const bool last_chunk = c + 1 == p.n_chunks, more = p.n_chunks > 1 && !(last_chunk && round + 1 == rounds);
-        // the next chunk, into the buffer that the barrier at the end of the previous chunk freed
-        if (more) stage_acts(a0, ac, last_chunk ? 0 : c + 1, buf ^ 1);
-        const uint32_t abase = smem + (uint32_t)(p.act_off + buf * p.act_buf);
-        const int j_end = nb - c * p.bpc < p.bpc ? nb - c * p.bpc : p.bpc;
-        for (int j = 0; j < j_end && live; ++j) {
-          fetch();
-          // groups newer than this step's weights: the stages - 1 fetches after it (a staged chunk among them only helps)
-          ib_wait(p.stages - 1);
-          __syncwarp();
-          const uint32_t st = wst + (uint32_t)step_stage * stage_bytes;
-          if (++step_stage == p.stages) step_stage = 0;
-          uint32_t k0 = 0, k1 = 0;
-          if constexpr (!F::kAligned) {  // rows past n repeat row n - 1
-            const int b = b_begin + c * p.bpc + j;
-            const int ra = tile * 16 + cx.gid < p.n ? tile * 16 + cx.gid : p.n - 1;
-            const int rb = tile * 16 + cx.gid + 8 < p.n ? tile * 16 + cx.gid + 8 : p.n - 1;
-            const uint32_t o = (uint32_t)gbase + (uint32_t)b * F::kBytes256;
-            k0 = (o + (uint32_t)ra * (uint32_t)p.row_bytes) & 15u, k1 = (o + (uint32_t)rb * (uint32_t)p.row_bytes) & 15u;
-          }
-          cx.r0 = st + (uint32_t)(cx.gid * F::kPitch) + k0;
-          cx.r1 = st + (uint32_t)((cx.gid + 8) * F::kPitch) + k1;
-          cx.lm = st + (uint32_t)(((lane & 7) + (lane & 8)) * F::kPitch) + 16u * (lane >> 4);
-          cx.act = abase + (uint32_t)((kpart * p.bpc + j) * slot_bytes);
-          F::template block<MT>(cx, facc);
-          __syncwarp();  // every lane has read the stage before any lane refills it
-        }
-        if (more) {
-          if (!p.act.rec) ib_wait(0);
-          __syncthreads();
-          buf ^= 1;
-          acts_landed(buf);
-        }
+    for (int pass = 0; pass < n_pass; ++pass) {
+      const int a0 = m_begin + pass * p.rows_cap;
+      const int ac = m_count - pass * p.rows_cap < p.rows_cap ? m_count - pass * p.rows_cap : p.rows_cap;
+      cx.nt = (ac + 7) >> 3;
+      if (pass > 0 || !first) __syncthreads();  // the previous pass's activations are done with
+      stage_acts(a0, ac, 0, 0);
+      if (!p.act.rec) {
+        ib_wait(0);
+        __syncthreads();
       }
-      // the shares' sums, two 8-row tiles at a time; a single share stores straight from its registers
-      const int row0 = tile * 16;
-      if (p.kp == 1) {
-        if (live) {
+      acts_landed(0);
+      int buf = 0;
+      for (int round = 0; round < rounds; ++round) {
+        float facc[MT][4];
 #pragma unroll
-          for (int mt = 0; mt < MT; ++mt)
+        for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              const int m = 8 * mt + 2 * cx.tig + (i & 1), col = cx.gid + 8 * (i >> 1);
-              if (m < ac && row0 + col < p.n) {
-                const int orow = p.out_rows ? p.out_rows[a0 + m] : a0 + m;
-                p.y[(size_t)orow * p.n + row0 + col] = facc[mt][i];
-              }
+          for (int i = 0; i < 4; ++i) facc[mt][i] = 0.f;
+        const int tile = t_begin + round * p.tg + slot;
+        const bool live = has_slot && tile < t_end;
+        for (int c = 0; c < n_chunks; ++c) {
+          const bool last_chunk = c + 1 == n_chunks, more = n_chunks > 1 && !(last_chunk && round + 1 == rounds);
+          // the next chunk, into the buffer that the barrier at the end of the previous chunk freed
+          if (more) stage_acts(a0, ac, last_chunk ? 0 : c + 1, buf ^ 1);
+          const uint32_t abase = smem + (uint32_t)(p.act_off + buf * p.act_buf);
+          const int j_end = nb - c * bpc < bpc ? nb - c * bpc : bpc;
+          for (int j = 0; j < j_end && live; ++j) {
+            fetch();
+            // groups newer than this step's weights: the stages - 1 fetches after it (a staged chunk among them only helps)
+            ib_wait(p.stages - 1);
+            __syncwarp();
+            const uint32_t st = wst + (uint32_t)step_stage * stage_bytes;
+            if (++step_stage == p.stages) step_stage = 0;
+            uint32_t k0 = 0, k1 = 0;
+            if constexpr (!F::kAligned) {  // rows past n repeat row n - 1
+              const int b = b_begin + c * bpc + j;
+              const int ra = tile * 16 + cx.gid < p.n ? tile * 16 + cx.gid : p.n - 1;
+              const int rb = tile * 16 + cx.gid + 8 < p.n ? tile * 16 + cx.gid + 8 : p.n - 1;
+              const uint32_t o = (uint32_t)gbase + (uint32_t)b * F::kBytes256;
+              k0 = (o + (uint32_t)ra * (uint32_t)p.row_bytes) & 15u, k1 = (o + (uint32_t)rb * (uint32_t)p.row_bytes) & 15u;
             }
-        }
-      } else {
-#pragma unroll
-        for (int m2 = 0; m2 < MT; m2 += 2) {
-          if (m2 < cx.nt) {
-            constexpr int kW = (MT > 1 ? 2 : 1) * 128;  // floats per warp
-            if (live) {
-#pragma unroll
-              for (int q = 0; q < (MT > 1 ? 2 : 1); ++q)
-#pragma unroll
-                for (int i = 0; i < 4; ++i) part[warp * kW + (q * 4 + i) * 32 + lane] = facc[m2 + q][i];
-            }
+            cx.r0 = st + (uint32_t)(cx.gid * F::kPitch) + k0;
+            cx.r1 = st + (uint32_t)((cx.gid + 8) * F::kPitch) + k1;
+            cx.lm = st + (uint32_t)(((lane & 7) + (lane & 8)) * F::kPitch) + 16u * (lane >> 4);
+            cx.act = abase + (uint32_t)((kpart * bpc + j) * slot_bytes);
+            F::template block<MT>(cx, facc);
+            __syncwarp();  // every lane has read the stage before any lane refills it
+          }
+          if (more) {
+            if (!p.act.rec) ib_wait(0);
             __syncthreads();
-            const int tiles_here = t_end - (t_begin + round * p.tg) < p.tg ? t_end - (t_begin + round * p.tg) : p.tg;
-            for (int i = threadIdx.x; i < tiles_here * kW; i += blockDim.x) {
-              const int ts = i / kW, o = i - ts * kW, ml = o >> 4, col = o & 15;
-              const int m = 8 * m2 + ml, gr = (t_begin + round * p.tg + ts) * 16 + col;
-              if (m < ac && gr < p.n) {
-                // fragment position of (activation row ml, weight row col)
-                const int src = (((ml >> 3) * 4 + ((ml & 1) | ((col >> 3) << 1))) << 5) + ((col & 7) << 2) + ((ml & 7) >> 1);
-                const float* q = part + (size_t)(ts * p.kp) * kW + src;
-                float sum = q[0];
-                for (int s = 1; s < p.kp; ++s) sum += q[s * kW];
-                const int orow = p.out_rows ? p.out_rows[a0 + m] : a0 + m;
-                p.y[(size_t)orow * p.n + gr] = sum;
-              }
-            }
-            __syncthreads();
+            buf ^= 1;
+            acts_landed(buf);
           }
         }
+        // the shares' sums, two 8-row tiles at a time; a single share stores straight from its registers
+        const int row0 = tile * 16;
+        if (p.kp == 1) {
+          if (live) {
+#pragma unroll
+            for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+              for (int i = 0; i < 4; ++i) {
+                const int m = 8 * mt + 2 * cx.tig + (i & 1), col = cx.gid + 8 * (i >> 1);
+                if (m < ac && row0 + col < p.n) {
+                  const int orow = kGrouped && p.out_rows ? p.out_rows[a0 + m] : a0 + m;
+                  p.y[(size_t)orow * p.n + row0 + col] = facc[mt][i];
+                }
+              }
+          }
+        } else {
+#pragma unroll
+          for (int m2 = 0; m2 < MT; m2 += 2) {
+            if (m2 < cx.nt) {
+              constexpr int kW = (MT > 1 ? 2 : 1) * 128;  // floats per warp
+              if (live) {
+#pragma unroll
+                for (int q = 0; q < (MT > 1 ? 2 : 1); ++q)
+#pragma unroll
+                  for (int i = 0; i < 4; ++i) part[warp * kW + (q * 4 + i) * 32 + lane] = facc[m2 + q][i];
+              }
+              __syncthreads();
+              const int tiles_here = t_end - (t_begin + round * p.tg) < p.tg ? t_end - (t_begin + round * p.tg) : p.tg;
+              for (int i = threadIdx.x; i < tiles_here * kW; i += blockDim.x) {
+                const int ts = i / kW, o = i - ts * kW, ml = o >> 4, col = o & 15;
+                const int m = 8 * m2 + ml, gr = (t_begin + round * p.tg + ts) * 16 + col;
+                if (m < ac && gr < p.n) {
+                  // fragment position of (activation row ml, weight row col)
+                  const int src = (((ml >> 3) * 4 + ((ml & 1) | ((col >> 3) << 1))) << 5) + ((col & 7) << 2) + ((ml & 7) >> 1);
+                  const float* q = part + (size_t)(ts * p.kp) * kW + src;
+                  float sum = q[0];
+                  for (int s = 1; s < p.kp; ++s) sum += q[s * kW];
+                  const int orow = kGrouped && p.out_rows ? p.out_rows[a0 + m] : a0 + m;
+                  p.y[(size_t)orow * p.n + gr] = sum;
+                }
+              }
+              __syncthreads();
+            }
+          }
+        }
       }
     }
+    if constexpr (!kGrouped) break;
+    ++grp, base += cost;
+    if (!segment()) break;
   }
 }
 
