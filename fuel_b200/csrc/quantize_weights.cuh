@@ -145,14 +145,70 @@ __global__ void __launch_bounds__(128) quantize_w_legacy32_kernel(const float* _
   }
 }
 
-// ---------------------------------------------------------------- Q4_K: one thread per 32-element sub-block
-// total order on floats (Rust total_cmp): only matters for -0.0 < +0.0 on finite data
-__device__ __forceinline__ bool qw_total_less(float a, float b) {
-  int ia = __float_as_int(a), ib = __float_as_int(b);
-  ia ^= (int)((unsigned)(ia >> 31) >> 1);
-  ib ^= (int)((unsigned)(ib >> 31) >> 1);
-  return ia < ib;
+// Smallest and largest in the total order on floats (Rust total_cmp; it differs from < on -0.0, +0.0 and NaN), by way of
+// integers in that order: the sign bit kept, the others flipped for negative values, which undoes itself.
+__device__ __forceinline__ int qw_ordered(int bits) { return bits ^ (int)((unsigned)(bits >> 31) >> 1); }
+template <int N>
+__device__ __forceinline__ void qw_total_min_max(const float (&v)[N], float& mn, float& mx) {
+  int lo = qw_ordered(__float_as_int(v[0])), hi = lo;
+#pragma unroll
+  for (int t = 1; t < N; ++t) {
+    const int o = qw_ordered(__float_as_int(v[t]));
+    lo = min(lo, o), hi = max(hi, o);
+  }
+  mn = __int_as_float(qw_ordered(lo)), mx = __int_as_float(qw_ordered(hi));
 }
+
+// roundf (halves away from zero), conversion to an integer (NaN to 0) and clamping to [0, nmax] for a small nmax, without the
+// conversions, which run at a quarter of the rate: clamped first, which changes nothing as the bounds are integers, then
+// floor(c + 0.5) from an addition that rounds down to a multiple of a half (4194304 = 2^22) and whose half is dropped.
+__device__ __forceinline__ uint32_t qw_level_bits(float r, float nmax) {
+  return __float_as_uint(__fadd_rd(fminf(fmaxf(r, 0.f), nmax), 4194304.5f)) & ~1u;
+}
+__device__ __forceinline__ float qw_level_float(uint32_t bits) { return __fsub_rn(__uint_as_float(bits), 4194304.f); }
+__device__ __forceinline__ uint32_t qw_level_int(uint32_t bits) { return (bits >> 1) & 0xffu; }
+
+// make_qkx1_quants(nmax, 5, x) (utils.rs:229-286): scale and minus the minimum. What bounds it is instructions, 14 per element
+// and sweep. The levels stay floats: as packed bytes, with conversions either way, converting 45 M elements to Q4_K took 246 us.
+template <int N>
+__device__ __forceinline__ void qw_make_qkx1(const float (&v)[N], float nmax, float& scale, float& negmin) {
+  scale = 0.f, negmin = 0.f;
+  float mn, mx;
+  qw_total_min_max(v, mn, mx);
+  if (mx != mn) {
+    if (mn > 0.f) mn = 0.f;
+    float iscale = __fdiv_rn(nmax, __fsub_rn(mx, mn));
+    scale = __fdiv_rn(1.0f, iscale);
+    float L[N];
+#pragma unroll
+    for (int t = 0; t < N; ++t) L[t] = 0.f;
+#pragma unroll 1
+    for (int it = 0; it < 5; ++it) {
+      float sumlx = 0.f, suml2 = 0.f;  // suml2: whole numbers below 2^24, exact
+      bool changed = false;
+#pragma unroll
+      for (int t = 0; t < N; ++t) {
+        const float xm = __fsub_rn(v[t], mn);
+        const float l = qw_level_float(qw_level_bits(__fmul_rn(iscale, xm), nmax));
+        changed |= l != L[t];
+        L[t] = l;
+        sumlx = __fadd_rn(sumlx, __fmul_rn(xm, l));
+        suml2 = __fmaf_rn(l, l, suml2);
+      }
+      scale = __fdiv_rn(sumlx, suml2);
+      float sum = 0.f;
+#pragma unroll
+      for (int t = 0; t < N; ++t) sum = __fadd_rn(sum, __fsub_rn(v[t], __fmul_rn(scale, L[t])));
+      mn = __fdiv_rn(sum, (float)N);
+      if (mn > 0.f) mn = 0.f;
+      iscale = __fdiv_rn(1.0f, scale);
+      if (!changed) break;
+    }
+    negmin = -mn;
+  }
+}
+
+// ---------------------------------------------------------------- Q4_K: one thread per 32-element sub-block
 
 // kFive: Q5_K (BlockQ5K::from_float, k_quants.rs:1732-1887): the same fit with 32 levels, the fifth bit of element t of
 // sub-block s kept as bit s of qh[t].
@@ -180,53 +236,8 @@ __global__ void __launch_bounds__(128) quantize_w_q4k_kernel(const float* __rest
 #pragma unroll
     for (int t = 0; t < 32; ++t) v[t] = 0.f;
   }
-  // make_qkx1_quants(nmax, 5, x) -> (scale, -min)
-  float scale = 0.f, negmin = 0.f;
-  {
-    float mn = v[0], mx = v[0];
-#pragma unroll
-    for (int t = 1; t < 32; ++t) {
-      if (qw_total_less(v[t], mn)) mn = v[t];
-      if (!qw_total_less(v[t], mx)) mx = v[t];
-    }
-    if (mx != mn) {
-      if (mn > 0.f) mn = 0.f;
-      float iscale = __fdiv_rn((float)kNmax, __fsub_rn(mx, mn));
-      scale = __fdiv_rn(1.0f, iscale);
-      uint32_t Lp[8];  // 32 levels, 4 bits used of each byte
-#pragma unroll
-      for (int t = 0; t < 8; ++t) Lp[t] = 0;
-      for (int it = 0; it < 5; ++it) {
-        float sumlx = 0.f;
-        int suml2 = 0;
-        bool changed = false;
-#pragma unroll
-        for (int t = 0; t < 32; ++t) {
-          const float xm = __fsub_rn(v[t], mn);
-          const int li = qw_clamp(qw_nearest_int(__fmul_rn(iscale, xm)), 0, kNmax);
-          const uint32_t old = (Lp[t >> 2] >> (8 * (t & 3))) & 0xff;
-          if ((uint32_t)li != old) {
-            Lp[t >> 2] = (Lp[t >> 2] & ~(0xffu << (8 * (t & 3)))) | ((uint32_t)li << (8 * (t & 3)));
-            changed = true;
-          }
-          sumlx = __fadd_rn(sumlx, __fmul_rn(xm, (float)li));
-          suml2 += li * li;
-        }
-        scale = __fdiv_rn(sumlx, (float)suml2);
-        float sum = 0.f;
-#pragma unroll
-        for (int t = 0; t < 32; ++t) {
-          const float li = (float)((Lp[t >> 2] >> (8 * (t & 3))) & 0xff);
-          sum = __fadd_rn(sum, __fsub_rn(v[t], __fmul_rn(scale, li)));
-        }
-        mn = __fdiv_rn(sum, 32.0f);
-        if (mn > 0.f) mn = 0.f;
-        iscale = __fdiv_rn(1.0f, scale);
-        if (!changed) break;
-      }
-      negmin = -mn;
-    }
-  }
+  float scale, negmin;
+  qw_make_qkx1(v, (float)kNmax, scale, negmin);
   // max over the eight sub-blocks, folded from 0 in index order (f32::max ignores NaN like fmaxf)
   float max_scale = 0.f, max_min = 0.f;
 #pragma unroll
@@ -256,8 +267,7 @@ __global__ void __launch_bounds__(128) quantize_w_q4k_kernel(const float* __rest
     const float dm = __fmul_rn(__half2float(hm), (float)lm);
 #pragma unroll
     for (int t = 0; t < 32; ++t) {
-      const int l = qw_clamp(qw_nearest_int(__fdiv_rn(__fadd_rn(v[t], dm), dsub)), 0, kNmax);
-      Lq[t >> 2] |= (uint32_t)l << (8 * (t & 3));
+      Lq[t >> 2] |= qw_level_int(qw_level_bits(__fdiv_rn(__fadd_rn(v[t], dm), dsub), (float)kNmax)) << (8 * (t & 3));
     }
   }
   // fifth bits: bit t of `high` says element t of this sub-block is above 15; every thread then holds all eight masks
@@ -361,47 +371,8 @@ __global__ void __launch_bounds__(128) quantize_w_q2k_kernel(const float* __rest
   const unsigned gmask = 0xffffu << base_lane;
   float v[16];
   qw_load16(x, sub, live, v);
-  // make_qkx1_quants(3, 5, x) -> (scale, -min)
-  float scale = 0.f, negmin = 0.f;
-  {
-    float mn = v[0], mx = v[0];
-#pragma unroll
-    for (int t = 1; t < 16; ++t) {
-      if (qw_total_less(v[t], mn)) mn = v[t];
-      if (!qw_total_less(v[t], mx)) mx = v[t];
-    }
-    if (mx != mn) {
-      if (mn > 0.f) mn = 0.f;
-      float iscale = __fdiv_rn(3.0f, __fsub_rn(mx, mn));
-      scale = __fdiv_rn(1.0f, iscale);
-      uint32_t Lp = 0;  // 16 levels, two bits each
-      for (int it = 0; it < 5; ++it) {
-        float sumlx = 0.f;
-        int suml2 = 0;
-        bool changed = false;
-#pragma unroll
-        for (int t = 0; t < 16; ++t) {
-          const float xm = __fsub_rn(v[t], mn);
-          const int li = qw_clamp(qw_nearest_int(__fmul_rn(iscale, xm)), 0, 3);
-          if ((uint32_t)li != ((Lp >> (2 * t)) & 3u)) {
-            Lp = (Lp & ~(3u << (2 * t))) | ((uint32_t)li << (2 * t));
-            changed = true;
-          }
-          sumlx = __fadd_rn(sumlx, __fmul_rn(xm, (float)li));
-          suml2 += li * li;
-        }
-        scale = __fdiv_rn(sumlx, (float)suml2);
-        float sum = 0.f;
-#pragma unroll
-        for (int t = 0; t < 16; ++t) sum = __fadd_rn(sum, __fsub_rn(v[t], __fmul_rn(scale, (float)((Lp >> (2 * t)) & 3u))));
-        mn = __fdiv_rn(sum, 16.0f);
-        if (mn > 0.f) mn = 0.f;
-        iscale = __fdiv_rn(1.0f, scale);
-        if (!changed) break;
-      }
-      negmin = -mn;
-    }
-  }
+  float scale, negmin;
+  qw_make_qkx1(v, 3.0f, scale, negmin);
   float max_scale = 0.f, max_min = 0.f;
 #pragma unroll
   for (int s2 = 0; s2 < 16; ++s2) {
@@ -425,7 +396,7 @@ __global__ void __launch_bounds__(128) quantize_w_q2k_kernel(const float* __rest
     const float dm = __fmul_rn(__half2float(hm), (float)(sc_byte >> 4));
 #pragma unroll
     for (int t = 0; t < 16; ++t)
-      lv |= (uint32_t)qw_clamp(qw_nearest_int(__fdiv_rn(__fadd_rn(v[t], dm), dsub)), 0, 3) << (2 * t);
+      lv |= qw_level_int(qw_level_bits(__fdiv_rn(__fadd_rn(v[t], dm), dsub), 3.0f)) << (2 * t);
   }
   uint8_t* ob = out + (live ? blk : 0) * Q2KL::kBytes;
   qw_store_qs2(lv, j, gmask, base_lane, live, ob + Q2KL::kOffQs);
