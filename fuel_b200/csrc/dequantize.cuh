@@ -76,11 +76,16 @@ __device__ __forceinline__ bool aligned16(const void* p) { return (reinterpret_c
 __device__ __forceinline__ uint32_t ldg_u16(const uint8_t* p) { return *reinterpret_cast<const uint16_t*>(p); }
 __device__ __forceinline__ uint32_t ldg_u32_2b(const uint8_t* p) { return ldg_u16(p) | (ldg_u16(p + 2) << 16); }
 
+// Every kernel here waits for its predecessor at its END: launched as a dependent of the activation conversion of the same
+// call (which starts its dependents only once everything before the call has finished) it runs beside it, and the GEMM
+// behind it still waits for both. In a plain launch the wait does nothing.
+
 // one thread per 16-byte nibble chunk: 16 low-nibble + 16 high-nibble elements
 template <typename T>
 __global__ void __launch_bounds__(256) dequant_q4k_kernel(const uint8_t* __restrict__ w, int64_t n_units, T* __restrict__ y) {
   const int64_t u = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (u >= n_units) return;
+  pdl_launch_dependents();
   const int64_t blk = u >> 3;
   const int cc = (int)(u & 7), g = cc >> 1, h = cc & 1;
   const uint8_t* b = w + blk * Q4KL::kBytes;
@@ -113,6 +118,7 @@ __global__ void __launch_bounds__(256) dequant_q4k_kernel(const uint8_t* __restr
   const bool vec = aligned16(y);
   store_run<T, 16>(out, lo, vec);
   store_run<T, 16>(out + 32, hi, vec);
+  pdl_wait();
 }
 
 // Q5_K (fuel-quantized/src/k_quants.rs:1889-1923): Q4_K's layout and scale packing plus a fifth bit per element in qh —
@@ -121,6 +127,7 @@ template <typename T>
 __global__ void __launch_bounds__(256) dequant_q5k_kernel(const uint8_t* __restrict__ w, int64_t n_units, T* __restrict__ y) {
   const int64_t u = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (u >= n_units) return;
+  pdl_launch_dependents();
   const int64_t blk = u >> 3;
   const int cc = (int)(u & 7), g = cc >> 1, h = cc & 1;
   const uint8_t* b = w + blk * Q5KL::kBytes;
@@ -155,6 +162,7 @@ __global__ void __launch_bounds__(256) dequant_q5k_kernel(const uint8_t* __restr
   const bool vec = aligned16(y);
   store_run<T, 16>(out, vlo, vec);
   store_run<T, 16>(out + 32, vhi, vec);
+  pdl_wait();
 }
 
 // one thread per four consecutive l of one 128-half: 16 elements
@@ -162,6 +170,7 @@ template <typename T>
 __global__ void __launch_bounds__(256) dequant_q6k_kernel(const uint8_t* __restrict__ w, int64_t n_units, T* __restrict__ y) {
   const int64_t u = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (u >= n_units) return;
+  pdl_launch_dependents();
   const int64_t blk = u >> 4;
   const int uu = (int)(u & 15), half = uu >> 3, l0 = (uu & 7) * 4;
   const uint8_t* b = w + blk * Q6KL::kBytes;
@@ -191,6 +200,7 @@ __global__ void __launch_bounds__(256) dequant_q6k_kernel(const uint8_t* __restr
   store_run<T, 4>(out + 32, v2, vec);
   store_run<T, 4>(out + 64, v3, vec);
   store_run<T, 4>(out + 96, v4, vec);
+  pdl_wait();
 }
 
 // one thread per 8 elements of a 32-block (4 threads per block)
@@ -198,6 +208,7 @@ template <typename T>
 __global__ void __launch_bounds__(256) dequant_q8_0_kernel(const uint8_t* __restrict__ w, int64_t n_units, T* __restrict__ y) {
   const int64_t u = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (u >= n_units) return;
+  pdl_launch_dependents();
   const int64_t blk = u >> 2;
   const int part = (int)(u & 3);
   const uint8_t* b = w + blk * Q8_0L::kBytes;
@@ -211,6 +222,7 @@ __global__ void __launch_bounds__(256) dequant_q8_0_kernel(const uint8_t* __rest
     o[2 * j + 1] = __fmul_rn((float)(int8_t)(v >> 8), d);
   }
   store_run<T, 8>(out, o, aligned16(y));
+  pdl_wait();
 }
 
 // one thread per 4 bytes of nibbles: elements 4p..4p+3 and 16+4p..
@@ -218,6 +230,7 @@ template <typename T>
 __global__ void __launch_bounds__(256) dequant_q4_0_kernel(const uint8_t* __restrict__ w, int64_t n_units, T* __restrict__ y) {
   const int64_t u = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (u >= n_units) return;
+  pdl_launch_dependents();
   const int64_t blk = u >> 2;
   const int part = (int)(u & 3);
   const uint8_t* b = w + blk * Q4_0L::kBytes;
@@ -234,6 +247,7 @@ __global__ void __launch_bounds__(256) dequant_q4_0_kernel(const uint8_t* __rest
   const bool vec = aligned16(y);
   store_run<T, 4>(out, lo, vec);
   store_run<T, 4>(out + 16, hi, vec);
+  pdl_wait();
 }
 
 // Q4_1 / Q5_0 / Q5_1 (k_quants.rs:354-374, 463-485, 578-602): one thread per 4 bytes of nibbles, elements 4p..4p+3
@@ -242,6 +256,7 @@ template <typename T, class L, bool kFive, bool kMin>
 __global__ void __launch_bounds__(256) dequant_legacy32_kernel(const uint8_t* __restrict__ w, int64_t n_units, T* __restrict__ y) {
   const int64_t u = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (u >= n_units) return;
+  pdl_launch_dependents();
   const int64_t blk = u >> 2;
   const int part = (int)(u & 3);
   const uint8_t* b = w + blk * L::kBytes;
@@ -264,6 +279,7 @@ __global__ void __launch_bounds__(256) dequant_legacy32_kernel(const uint8_t* __
   const bool vec = aligned16(y);
   store_run<T, 4>(out, lo, vec);
   store_run<T, 4>(out + 16, hi, vec);
+  pdl_wait();
 }
 // Q2_K (k_quants.rs:958-994): y = (d * sc_lo) * q - dmin * sc_hi; Q3_K (:1314-1366): y = (d * (sc - 32)) * q with
 // q = low two bits - (high bit set ? 0 : 4). One thread per 4 bytes of qs of one bit pair: 4 elements.
@@ -271,6 +287,7 @@ template <typename T>
 __global__ void __launch_bounds__(256) dequant_q2k_kernel(const uint8_t* __restrict__ w, int64_t n_units, T* __restrict__ y) {
   const int64_t u = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (u >= n_units) return;
+  pdl_launch_dependents();
   const int64_t blk = u >> 6;
   const int e0 = (int)(u & 63) * 4;                       // first of four consecutive elements
   const int c = e0 >> 7, j = (e0 >> 5) & 3, bb = e0 & 31;  // chunk, bit pair, byte within the chunk's 32
@@ -284,11 +301,13 @@ __global__ void __launch_bounds__(256) dequant_q2k_kernel(const uint8_t* __restr
 #pragma unroll
   for (int t = 0; t < 4; ++t) o[t] = __fsub_rn(__fmul_rn(dl, (float)((v >> (8 * t + 2 * j)) & 3u)), ml);
   store_run<T, 4>(out, o, aligned16(y));
+  pdl_wait();
 }
 template <typename T>
 __global__ void __launch_bounds__(256) dequant_q3k_kernel(const uint8_t* __restrict__ w, int64_t n_units, T* __restrict__ y) {
   const int64_t u = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (u >= n_units) return;
+  pdl_launch_dependents();
   const int64_t blk = u >> 6;
   const int e0 = (int)(u & 63) * 4;
   const int c = e0 >> 7, j = (e0 >> 5) & 3, bb = e0 & 31, is = e0 >> 4;
@@ -306,6 +325,7 @@ __global__ void __launch_bounds__(256) dequant_q3k_kernel(const uint8_t* __restr
     o[t] = __fmul_rn(dl, (float)q);
   }
   store_run<T, 4>(out, o, aligned16(y));
+  pdl_wait();
 }
 
 // Q8_K blocks back to f32 (x.d * q, k_quants.rs:2269-2280); one thread per 4 elements
@@ -313,6 +333,7 @@ template <typename T>
 __global__ void __launch_bounds__(256) dequant_q8k_kernel(const uint8_t* __restrict__ w, int64_t n_units, T* __restrict__ y) {
   const int64_t u = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (u >= n_units) return;
+  pdl_launch_dependents();
   const int64_t blk = u >> 6;
   const int part = (int)(u & 63);
   const uint8_t* b = w + blk * Q8KL::kBytes;
@@ -323,6 +344,7 @@ __global__ void __launch_bounds__(256) dequant_q8k_kernel(const uint8_t* __restr
 #pragma unroll
   for (int t = 0; t < 4; ++t) o[t] = __fmul_rn(d, (float)(int8_t)((v >> (8 * t)) & 0xff));
   store_run<T, 4>(out, o, aligned16(y));
+  pdl_wait();
 }
 
 }  // namespace fq

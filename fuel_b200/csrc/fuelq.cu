@@ -79,7 +79,7 @@ bool supported_weight(int t) {
 // kernels of a call always may: its first kernel lets them start only after its own wait, see quantize_q8k_kernel's
 // `late_trigger`).
 template <typename... KArgs, typename... Args>
-cudaError_t launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args) {
+cudaError_t launch_if(bool dependent, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = block;
@@ -89,8 +89,12 @@ cudaError_t launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = dependent ? 1 : 0;
   return cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...);
+}
+template <typename... KArgs, typename... Args>
+cudaError_t launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args) {
+  return launch_if(true, kernel, grid, block, smem, stream, args...);
 }
 
 // ------------------------------------------------------------------ activation quantization
@@ -739,7 +743,8 @@ int32_t decode_chunked(int type, int64_t m_total, int64_t n, int64_t k, const vo
 // out_type: kF32, kF16, kBF16, or the tensor-core path's operands: kF16Sat (f16 with finite overflow saturated) and
 // kTf32 (f32 rounded to tf32)
 constexpr int kF16Sat = -16, kTf32Out = -32;
-int32_t dequantize_impl(int ggml_type, int64_t numel, const void* blocks, void* y, int out_type, cudaStream_t stream) {
+int32_t dequantize_impl(int ggml_type, int64_t numel, const void* blocks, void* y, int out_type, cudaStream_t stream,
+                        bool dependent = false) {
   const int be = block_elems(ggml_type);
   if (be == 0) return kNotSupported;
   if (numel < 0 || numel % be) return kInvalidProblem;
@@ -759,19 +764,20 @@ int32_t dequantize_impl(int ggml_type, int64_t numel, const void* blocks, void* 
     case kQ8K: case kQ2K: case kQ3K: units = nb * 64; break;
     default: return kNotSupported;
   }
+  cudaError_t e = cudaSuccess;
   const dim3 block(256), grid((unsigned)((units + 255) / 256));
 #define FQ_DEQ(KERNEL)                                                                        \
   do {                                                                                        \
     if (out_type == kF32)                                                                     \
-      KERNEL<float><<<grid, block, 0, stream>>>(w, units, (float*)y);                         \
+      e = launch_if(dependent, KERNEL<float>, grid, block, 0, stream, w, units, (float*)y); \
     else if (out_type == kF16)                                                                \
-      KERNEL<__half><<<grid, block, 0, stream>>>(w, units, (__half*)y);                       \
+      e = launch_if(dependent, KERNEL<__half>, grid, block, 0, stream, w, units, (__half*)y); \
     else if (out_type == kF16Sat)                                                             \
-      KERNEL<half_sat><<<grid, block, 0, stream>>>(w, units, (half_sat*)y);                   \
+      e = launch_if(dependent, KERNEL<half_sat>, grid, block, 0, stream, w, units, (half_sat*)y); \
     else if (out_type == kTf32Out)                                                            \
-      KERNEL<f32_tf32><<<grid, block, 0, stream>>>(w, units, (f32_tf32*)y);                   \
+      e = launch_if(dependent, KERNEL<f32_tf32>, grid, block, 0, stream, w, units, (f32_tf32*)y); \
     else                                                                                      \
-      KERNEL<__nv_bfloat16><<<grid, block, 0, stream>>>(w, units, (__nv_bfloat16*)y);         \
+      e = launch_if(dependent, KERNEL<__nv_bfloat16>, grid, block, 0, stream, w, units, (__nv_bfloat16*)y); \
   } while (0)
   switch (ggml_type) {
     case kQ4K: FQ_DEQ(dequant_q4k_kernel); break;
@@ -782,15 +788,15 @@ int32_t dequantize_impl(int ggml_type, int64_t numel, const void* blocks, void* 
 #define FQ_DEQ_L(L, FIVE, MIN)                                                                                  \
   do {                                                                                                          \
     if (out_type == kF32)                                                                                       \
-      dequant_legacy32_kernel<float, L, FIVE, MIN><<<grid, block, 0, stream>>>(w, units, (float*)y);            \
+      e = launch_if(dependent, dequant_legacy32_kernel<float, L, FIVE, MIN>, grid, block, 0, stream, w, units, (float*)y); \
     else if (out_type == kF16)                                                                                  \
-      dequant_legacy32_kernel<__half, L, FIVE, MIN><<<grid, block, 0, stream>>>(w, units, (__half*)y);          \
+      e = launch_if(dependent, dequant_legacy32_kernel<__half, L, FIVE, MIN>, grid, block, 0, stream, w, units, (__half*)y); \
     else if (out_type == kF16Sat)                                                                               \
-      dequant_legacy32_kernel<half_sat, L, FIVE, MIN><<<grid, block, 0, stream>>>(w, units, (half_sat*)y);      \
+      e = launch_if(dependent, dequant_legacy32_kernel<half_sat, L, FIVE, MIN>, grid, block, 0, stream, w, units, (half_sat*)y); \
     else if (out_type == kTf32Out)                                                                              \
-      dequant_legacy32_kernel<f32_tf32, L, FIVE, MIN><<<grid, block, 0, stream>>>(w, units, (f32_tf32*)y);      \
+      e = launch_if(dependent, dequant_legacy32_kernel<f32_tf32, L, FIVE, MIN>, grid, block, 0, stream, w, units, (f32_tf32*)y); \
     else                                                                                                        \
-      dequant_legacy32_kernel<__nv_bfloat16, L, FIVE, MIN><<<grid, block, 0, stream>>>(w, units, (__nv_bfloat16*)y); \
+      e = launch_if(dependent, dequant_legacy32_kernel<__nv_bfloat16, L, FIVE, MIN>, grid, block, 0, stream, w, units, (__nv_bfloat16*)y); \
   } while (0)
     case kQ4_1: FQ_DEQ_L(Q4_1L, false, true); break;
     case kQ5_0: FQ_DEQ_L(Q5_0L, true, false); break;
@@ -801,7 +807,7 @@ int32_t dequantize_impl(int ggml_type, int64_t numel, const void* blocks, void* 
     case kQ3K: FQ_DEQ(dequant_q3k_kernel); break;
   }
 #undef FQ_DEQ
-  return cudaGetLastError() == cudaSuccess ? kOk : kLaunchFailure;
+  return e == cudaSuccess ? kOk : kLaunchFailure;
 }
 
 
@@ -913,9 +919,7 @@ cudaError_t launch_plain_gemm_t(PlainGemmParams p, const void* xb, const void* w
     if (e != cudaSuccess) return e;
     attr_set[dev] = true;
   }
-  CUtensorMap xmap, wmap;
-  if (!make_x_map(xb, p.M, p.K, kTileM, kTf32, kF16, &xmap)) return cudaErrorUnknown;
-  if (!make_x_map(w, p.N, p.K, kPfTileN, kTf32, kF16, &wmap)) return cudaErrorUnknown;
+  CUtensorMap xmap, xmap_piece, wmap;
   // Work items: whole tiles for the full rounds of thread blocks; the tiles of a last, partly filled round are cut along M
   // into 2 or 4 pieces (at least 64 activation rows each) while the pieces still fit one round.
   const int tiles_n = (p.N + kPfTileN - 1) / kPfTileN;
@@ -932,9 +936,11 @@ cudaError_t launch_plain_gemm_t(PlainGemmParams p, const void* xb, const void* w
   p.whole_tiles = (int)whole;
   p.split_log2 = split;
   p.n_items = (int)items;
+  if (!make_x_map(xb, p.M, p.K, kTileM, kTf32, kF16, &xmap)) return cudaErrorUnknown;
+  if (!make_x_map(xb, p.M, p.K, kTileM >> split, kTf32, kF16, &xmap_piece)) return cudaErrorUnknown;
+  if (!make_x_map(w, p.N, p.K, kPfTileN, kTf32, kF16, &wmap)) return cudaErrorUnknown;
   const unsigned grid = (unsigned)(items < sm_count ? items : sm_count);
-  kern<<<grid, kPgThreads, smem, stream>>>(p, xmap, wmap);
-  return cudaGetLastError();
+  return launch(kern, dim3(grid), dim3(kPgThreads), smem, stream, p, xmap, xmap_piece, wmap);
 }
 
 // type < 0: `w` is a slab of rows already in the operand type (plain_gemm.cuh); else GGUF blocks dequantized inside the
@@ -1004,23 +1010,23 @@ int32_t prefill_impl(int type, int64_t m, int64_t n, int64_t k, const void* w, c
   void* xb = workspace;  // the activations in the tensor cores' operand type: f16 (rows scaled), bf16, or f32 rounded to tf32
   float* unscale = (float*)((uint8_t*)workspace + align_up((size_t)m * k * (tf32 ? 4 : 2), 256));
   const int64_t n4 = m * k / 4;
-  if (tf32)
-    f32_to_tf32_kernel<<<(unsigned)((n4 + 255) / 256), 256, 0, stream>>>(x, n4, (float*)xb);
-  else if (f16)
-    f32_to_f16_rows_kernel<<<(unsigned)m, 256, 0, stream>>>(x, (int)k, (__half*)xb, unscale);
-  else
-    f32_to_bf16_kernel<<<(unsigned)((n4 + 255) / 256), 256, 0, stream>>>(x, n4, (__nv_bfloat16*)xb);
-  if (cudaGetLastError() != cudaSuccess) return kLaunchFailure;
+  const unsigned wide_grid = (unsigned)((n4 + 255) / 256);
+  const cudaError_t e = tf32  ? launch(f32_to_tf32_kernel, dim3(wide_grid), dim3(256), 0, stream, x, n4, (float*)xb)
+                        : f16 ? launch(f32_to_f16_rows_kernel, dim3((unsigned)m), dim3(256), 0, stream, x, (int)k, (__half*)xb, unscale)
+                              : launch(f32_to_bf16_kernel, dim3(wide_grid), dim3(256), 0, stream, x, n4, (__nv_bfloat16*)xb);
+  if (e != cudaSuccess) return kLaunchFailure;
   if (one_kernel || !prefill_uses_slab(type, m)) return prefill_gemm(type, m, n, k, w, y_dst, n_dst, ldy, n_off, workspace, stream);
   // Dequantize a slab of rows into the operand type (the reference's to_float values in f32, then one rounding), multiply
-  // it, take the next slab. Kernels on one stream, so the slab is reused.
+  // it, take the next slab. Kernels on one stream, so the slab is reused. The first slab is dequantized beside the conversion
+  // of the activations (which lets it start once everything before the call has finished, and which it waits for at its
+  // end); a later one overwrites what the GEMM before it reads, and is launched plainly.
   uint8_t* slab = (uint8_t*)workspace + prefill_x_bytes(m, k);
   const int64_t slab_rows = prefill_slab_rows(n, k);
   const int64_t row_bytes = k / block_elems(type) * block_bytes(type);
   const int out_type = tf32 ? kTf32Out : f16 ? kF16Sat : (int)kBF16;
   for (int64_t r0 = 0; r0 < n; r0 += slab_rows) {
     const int64_t rows = n - r0 < slab_rows ? n - r0 : slab_rows;
-    int32_t st = dequantize_impl(type, rows * k, (const uint8_t*)w + r0 * row_bytes, slab, out_type, stream);
+    int32_t st = dequantize_impl(type, rows * k, (const uint8_t*)w + r0 * row_bytes, slab, out_type, stream, r0 == 0);
     if (st != kOk) return st;
     st = prefill_gemm(-1, m, rows, k, slab, y_dst, n_dst, ldy, n_off + r0, workspace, stream);
     if (st != kOk) return st;
@@ -1540,7 +1546,8 @@ int32_t fuelq_moe_route(const float* logits, int64_t n_tokens, int32_t n_experts
   if (n_tokens == 0) return kOk;
   if (n_tokens > (1 << 24)) return kNotSupported;
   if (!logits || !topk_ids || !topk_weights) return kInvalidProblem;
-  const cudaError_t e = launch(moe_route_kernel, dim3((unsigned)((n_tokens + 7) / 8)), dim3(256), 0, (cudaStream_t)stream,
+  const auto kern = n_experts <= 64 ? moe_route_kernel<2> : n_experts <= 128 ? moe_route_kernel<4> : moe_route_kernel<32>;
+  const cudaError_t e = launch(kern, dim3((unsigned)((n_tokens + 7) / 8)), dim3(256), 0, (cudaStream_t)stream,
                                logits, (int)n_tokens, (int)n_experts, (int)top_k, (int*)topk_ids, topk_weights);
   return e == cudaSuccess ? kOk : kLaunchFailure;
 }
@@ -1734,7 +1741,9 @@ int32_t fuelq_moe_combine(const float* y_pairs, const int32_t* topk_ids, const f
     return kInvalidProblem;
   if (n_tokens == 0) return kOk;
   if (!y_pairs || !topk_ids || !topk_weights || !out) return kInvalidProblem;
-  const cudaError_t e = launch(moe_combine_kernel, dim3((unsigned)n_tokens), dim3(256), 0, (cudaStream_t)stream, y_pairs,
+  // a few tokens: their columns over several thread blocks
+  const unsigned parts = n_tokens >= 148 ? 1 : (unsigned)((n + 1023) / 1024 < 16 ? (n + 1023) / 1024 : 16);
+  const cudaError_t e = launch(moe_combine_kernel, dim3((unsigned)n_tokens, parts), dim3(256), 0, (cudaStream_t)stream, y_pairs,
                                (const int*)topk_ids, topk_weights, (int)top_k, (int)n, out);
   return e == cudaSuccess ? kOk : kLaunchFailure;
 }

@@ -13,8 +13,8 @@
 //                      activation rows' power-of-two scaling here).
 // Work items are the 128 x kTileM output tiles in an order that keeps the thread blocks of one round on the same few weight
 // rows (M fastest). When the tiles do not fill a last round of thread blocks, the tiles of that round are cut along M into
-// 2 or 4 pieces (same loads, narrower MMAs), so the round takes a half or a quarter of a tile's time instead of a
-// whole one. Every wait is bounded; on expiry the block raises an abort flag, lets its copies land, frees its tensor
+// 2 or 4 pieces (narrower MMAs, and copies of their own activations alone), so the round takes a half or a
+// quarter of a tile's time instead of a whole one. Every wait is bounded; on expiry the block raises an abort flag, lets its copies land, frees its tensor
 // memory and returns.
 #pragma once
 #include "prefill.cuh"
@@ -48,8 +48,8 @@ struct PlainGemmSmem {
 };
 
 struct PgItem {
-  int n0, m0;    // first weight row, first activation row of the TILE (what is loaded)
-  int col, width;  // the piece: activation rows m0 + col .. m0 + col + width of it (what is multiplied and stored)
+  int n0, m0;  // first weight row, first activation row
+  int width;   // activation rows, a multiple of 32
 };
 __device__ __forceinline__ PgItem pg_item(const PlainGemmParams& p, int i, int tile_m) {
   int tile, col = 0, width = tile_m;
@@ -65,11 +65,12 @@ __device__ __forceinline__ PgItem pg_item(const PlainGemmParams& p, int i, int t
   // activation rows past M need no products: narrow the piece to the next multiple of 32 rows (possibly to nothing)
   const int left = p.M - (tm * tile_m + col);
   if (left < width) width = left <= 0 ? 0 : (left + 31) & ~31;
-  return PgItem{tn * kPfTileN, tm * tile_m, col, width};
+  return PgItem{tn * kPfTileN, tm * tile_m + col, width};
 }
 
 template <int kTileM, int kStages, bool kTf32, bool kF16, bool kMulti>
 __global__ void __launch_bounds__(kPgThreads, 1) plain_gemm_kernel(const PlainGemmParams p, const __grid_constant__ CUtensorMap xmap,
+                                                                   const __grid_constant__ CUtensorMap xmap_piece,
                                                                    const __grid_constant__ CUtensorMap wmap) {
   extern __shared__ __align__(1024) uint8_t pg_smem[];
   constexpr int kWBytes = kPfTileN * 128, kXBytes = kTileM * 128, kStageBytes = kWBytes + kXBytes;
@@ -100,6 +101,7 @@ __global__ void __launch_bounds__(kPgThreads, 1) plain_gemm_kernel(const PlainGe
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  pdl_wait();
   const uint32_t tmem_d = *reinterpret_cast<volatile uint32_t*>(&sm->tmem_base);
   volatile int* abort_flag = &sm->abort_flag;
 
@@ -111,19 +113,22 @@ __global__ void __launch_bounds__(kPgThreads, 1) plain_gemm_kernel(const PlainGe
       for (int i = blockIdx.x; i < p.n_items && !*abort_flag; i += gridDim.x) {
         const PgItem w = pg_item(p, i, kTileM);
         if (w.width == 0) continue;  // every role skips the same items
+        const CUtensorMap* map = i < p.whole_tiles ? &xmap : &xmap_piece;
+        const int rows = i < p.whole_tiles ? kTileM : kTileM >> p.split_log2;
         for (int it = 0; it < n_iter && !*abort_flag; ++it) {
           if (issued >= kStages && !mbar_wait_bounded(&sm->empty[s], ph ^ 1u)) {
             record_dev_error(kErrEmptyWait);
             *abort_flag = 1;
             break;
           }
-          mbar_arrive_expect_tx(&sm->full[s], (uint32_t)kStageBytes);
+          mbar_arrive_expect_tx(&sm->full[s], (uint32_t)(kWBytes + rows * 128));
           tma_load_2d(base_u32 + s * kStageBytes, &wmap, it * kStageK, w.n0, &sm->full[s]);
-          tma_load_2d(base_u32 + s * kStageBytes + kWBytes, &xmap, it * kStageK, w.m0, &sm->full[s]);
+          tma_load_2d(base_u32 + s * kStageBytes + kWBytes, map, it * kStageK, w.m0, &sm->full[s]);
           ++issued;
           if (++s == kStages) s = 0, ph ^= 1u;
         }
       }
+      pdl_launch_dependents();  // all that is left is a tile's worth of products: waiting blocks earlier than this cost 2 %
       if (*abort_flag) {  // leaving early: let the copies already issued land first
         for (int g = (issued > kStages ? issued - kStages : 0); g < issued; ++g)
           if (!mbar_wait_bounded(&sm->full[g % kStages], (g / kStages) & 1)) record_dev_error(kErrDrainWait);
@@ -156,7 +161,7 @@ __global__ void __launch_bounds__(kPgThreads, 1) plain_gemm_kernel(const PlainGe
             break;
           }
           tc_fence_after();
-          const uint32_t a_addr = base_u32 + s * kStageBytes, b_addr = a_addr + kWBytes + (uint32_t)w.col * 128u;
+          const uint32_t a_addr = base_u32 + s * kStageBytes, b_addr = a_addr + kWBytes;
 #pragma unroll
           for (int kk = 0; kk < 4; ++kk) {  // 32 bytes along K per instruction: 16 16-bit values or 8 tf32
             if constexpr (kTf32)
@@ -204,7 +209,7 @@ __global__ void __launch_bounds__(kPgThreads, 1) plain_gemm_kernel(const PlainGe
       for (int c = 0; c < chunks; ++c) {
         uint32_t v[32];
         tmem_ld32(tmem_d + ((uint32_t)(q * 32) << 16) + (uint32_t)(b * kTileM + c * 32), v);
-        const int mbase = w.m0 + w.col + c * 32;
+        const int mbase = w.m0 + c * 32;
         if constexpr (kF16) {  // undo the scaling of activation row mbase + j (a power of two: exact)
           const int ml = mbase + lane;
           const float mine = ml < p.M ? p.row_unscale[ml] : 1.0f;

@@ -634,6 +634,8 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_gemm_kernel(const Prefi
 
 // f32 -> f32 rounded to tf32 (activation pre-pass of the tf32 form)
 __global__ void __launch_bounds__(256) f32_to_tf32_kernel(const float* x, int64_t n4, float* y) {
+  pdl_wait();
+  pdl_launch_dependents();
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n4) {
     const float4 v = reinterpret_cast<const float4*>(x)[i];
@@ -646,8 +648,9 @@ __global__ void __launch_bounds__(256) f32_to_tf32_kernel(const float* x, int64_
 // f32 -> f16 activation pre-pass, one thread block per row: the row is scaled by the power of two that brings its
 // largest magnitude into [2^13, 2^14) (exact; keeps large rows finite and small rows out of the subnormals), and
 // unscale[row] holds the inverse for the epilogue. Rows of zeros or with non-finite values are left unscaled.
-__global__ void __launch_bounds__(256) f32_to_f16_rows_kernel(const float* __restrict__ x, int K, __half* __restrict__ y,
-                                                              float* __restrict__ unscale) {
+__global__ void __launch_bounds__(256) f32_to_f16_rows_kernel(const float* x, int K, __half* y, float* unscale) {
+  pdl_wait();
+  pdl_launch_dependents();
   __shared__ float red[8];
   const float4* src = reinterpret_cast<const float4*>(x + (size_t)blockIdx.x * K);
   const int n4 = K >> 2;
@@ -684,7 +687,9 @@ __global__ void __launch_bounds__(256) f32_to_f16_rows_kernel(const float* __res
 }
 
 // f32 -> bf16 activation pre-pass
-__global__ void __launch_bounds__(256) f32_to_bf16_kernel(const float* __restrict__ x, int64_t n4, __nv_bfloat16* __restrict__ y) {
+__global__ void __launch_bounds__(256) f32_to_bf16_kernel(const float* x, int64_t n4, __nv_bfloat16* y) {
+  pdl_wait();
+  pdl_launch_dependents();
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n4) return;
   const float4 v = reinterpret_cast<const float4*>(x)[i];
