@@ -22,9 +22,10 @@
 namespace fq {
 
 constexpr float kMoeMaskNeg = -1.0e30f;  // fuel-core/src/lazy_nn/moe.rs:28
-constexpr int kMoeMaxTopK = 16;
+constexpr int kMoeMaxTopK = 16;  // a power of two, at most the lanes of a warp
 
 // ---- router: one warp per token, n_experts <= 1024 -------------------------------------------
+template <int kPer>
 __global__ void __launch_bounds__(256) moe_route_kernel(const float* logits, int n_tokens, int n_experts, int top_k,
                                                         int* topk_ids, float* topk_w) {
   pdl_launch_dependents();
@@ -32,23 +33,20 @@ __global__ void __launch_bounds__(256) moe_route_kernel(const float* logits, int
   const int lane = threadIdx.x & 31;
   const int t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (t >= n_tokens) return;
-  float v[32];  // this lane's logits: experts lane, lane + 32, ...
-  const int per = (n_experts + 31) >> 5;
+  float v[kPer];  // this lane's logits: experts lane, lane + 32, ...
 #pragma unroll
-  for (int j = 0; j < 32; ++j) {
+  for (int j = 0; j < kPer; ++j) {
     const int e = lane + 32 * j;
-    v[j] = (j < per && e < n_experts) ? logits[(size_t)t * n_experts + e] : -INFINITY;
+    v[j] = e < n_experts ? logits[(size_t)t * n_experts + e] : -INFINITY;
   }
-  float picked[kMoeMaxTopK];
+  float picked = 0.f;  // lane r's: the logit of the r-th choice
   for (int r = 0; r < top_k; ++r) {
     float bv = -INFINITY;
     int bi = 0x7fffffff;
 #pragma unroll
-    for (int j = 0; j < 32; ++j) {
-      if (j < per) {
-        const int e = lane + 32 * j;
-        if (e < n_experts && (v[j] > bv || (v[j] == bv && e < bi))) bv = v[j], bi = e;  // first maximum wins
-      }
+    for (int j = 0; j < kPer; ++j) {
+      const int e = lane + 32 * j;
+      if (e < n_experts && (v[j] > bv || (v[j] == bv && e < bi))) bv = v[j], bi = e;  // first maximum wins
     }
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) {
@@ -56,24 +54,19 @@ __global__ void __launch_bounds__(256) moe_route_kernel(const float* logits, int
       const int oi = __shfl_xor_sync(0xffffffffu, bi, off);
       if (ov > bv || (ov == bv && oi < bi)) bv = ov, bi = oi;
     }
-    picked[r] = bv;
+    if (lane == r) picked = bv;
     if (lane == 0) topk_ids[(size_t)t * top_k + r] = bi;
 #pragma unroll
-    for (int j = 0; j < 32; ++j)
-      if (j < per && lane + 32 * j == bi) v[j] = __fadd_rn(v[j], kMoeMaskNeg);  // scatter_add of the mask value
+    for (int j = 0; j < kPer; ++j)
+      if (lane + 32 * j == bi) v[j] = __fadd_rn(v[j], kMoeMaskNeg);  // scatter_add of the mask value
   }
-  if (lane == 0) {
-    float mx = picked[0];
-    for (int r = 1; r < top_k; ++r)
-      if (picked[r] > mx) mx = picked[r];
-    float sum = 0.f;
-    for (int r = 0; r < top_k; ++r) {
-      picked[r] = expf(picked[r] - mx);
-      sum = __fadd_rn(sum, picked[r]);
-    }
-    const float inv = 1.0f / sum;
-    for (int r = 0; r < top_k; ++r) topk_w[(size_t)t * top_k + r] = __fmul_rn(picked[r], inv);
-  }
+  float mx = lane < top_k ? picked : -INFINITY;
+#pragma unroll
+  for (int off = kMoeMaxTopK / 2; off > 0; off >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
+  const float p = expf(picked - mx);
+  float sum = 0.f;
+  for (int r = 0; r < top_k; ++r) sum = __fadd_rn(sum, __shfl_sync(0xffffffffu, p, r));  // in order of choice
+  if (lane < top_k) topk_w[(size_t)t * top_k + lane] = __fmul_rn(p, 1.0f / sum);
 }
 
 // ---- bucketing: pairs (token * top_k + slot) sorted by expert, ascending pair id inside an expert.
@@ -473,38 +466,42 @@ __global__ void __launch_bounds__(256) moe_combine_kernel(const float* y_pairs, 
   pdl_launch_dependents();
   pdl_wait();
   const int t = blockIdx.x;
-  if (threadIdx.x == 0) {
-    int ord[kMoeMaxTopK];
-    for (int s = 0; s < top_k; ++s) ord[s] = s;
-    for (int a = 1; a < top_k; ++a) {  // insertion sort of the slots by expert id (ids are distinct)
-      const int sa = ord[a], ea = topk_ids[(size_t)t * top_k + sa];
-      int b = a - 1;
-      while (b >= 0 && topk_ids[(size_t)t * top_k + ord[b]] > ea) {
-        ord[b + 1] = ord[b];
-        --b;
-      }
-      ord[b + 1] = sa;
+  if (threadIdx.x < 32) {  // the slots by expert id: a slot's place is the number of slots that come before it
+    const int lane = threadIdx.x, id = lane < top_k ? topk_ids[(size_t)t * top_k + lane] : 0;
+    const float w = lane < top_k ? topk_w[(size_t)t * top_k + lane] : 0.f;
+    int place = 0;
+    for (int s = 0; s < top_k; ++s) {
+      const int other = __shfl_sync(0xffffffffu, id, s);
+      place += other < id || (other == id && s < lane);
     }
-    for (int s = 0; s < top_k; ++s) ord_s[s] = ord[s], w_s[s] = topk_w[(size_t)t * top_k + ord[s]];
+    if (lane < top_k) ord_s[place] = lane, w_s[place] = w;
   }
   __syncthreads();
   const float* base = y_pairs + (size_t)t * top_k * n;
   if ((n & 3) == 0 && (reinterpret_cast<uintptr_t>(y_pairs) & 15) == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0) {
-    for (int c = threadIdx.x; c < (n >> 2); c += blockDim.x) {
+    for (int c = blockIdx.y * blockDim.x + threadIdx.x; c < (n >> 2); c += gridDim.y * blockDim.x) {
       float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-      for (int s = 0; s < top_k; ++s) {
-        const float4 v = reinterpret_cast<const float4*>(base + (size_t)ord_s[s] * n)[c];
-        const float w = w_s[s];
-        acc.x = __fadd_rn(acc.x, __fmul_rn(v.x, w));  // scale, then add: two roundings
-        acc.y = __fadd_rn(acc.y, __fmul_rn(v.y, w));
-        acc.z = __fadd_rn(acc.z, __fmul_rn(v.z, w));
-        acc.w = __fadd_rn(acc.w, __fmul_rn(v.w, w));
+      for (int s0 = 0; s0 < top_k; s0 += 4) {  // four slots' loads in flight
+        float4 v[4];
+#pragma unroll
+        for (int s = 0; s < 4; ++s)
+          if (s0 + s < top_k) v[s] = reinterpret_cast<const float4*>(base + (size_t)ord_s[s0 + s] * n)[c];
+#pragma unroll
+        for (int s = 0; s < 4; ++s) {
+          if (s0 + s < top_k) {
+            const float w = w_s[s0 + s];
+            acc.x = __fadd_rn(acc.x, __fmul_rn(v[s].x, w));  // scale, then add: two roundings
+            acc.y = __fadd_rn(acc.y, __fmul_rn(v[s].y, w));
+            acc.z = __fadd_rn(acc.z, __fmul_rn(v[s].z, w));
+            acc.w = __fadd_rn(acc.w, __fmul_rn(v[s].w, w));
+          }
+        }
       }
       reinterpret_cast<float4*>(out + (size_t)t * n)[c] = acc;
     }
     return;
   }
-  for (int c = threadIdx.x; c < n; c += blockDim.x) {
+  for (int c = blockIdx.y * blockDim.x + threadIdx.x; c < n; c += gridDim.y * blockDim.x) {
     float acc = 0.f;
     for (int s = 0; s < top_k; ++s) acc = __fadd_rn(acc, __fmul_rn(base[(size_t)ord_s[s] * n + c], w_s[s]));
     out[(size_t)t * n + c] = acc;
