@@ -654,19 +654,23 @@ int32_t ibatch_fmt(int n_groups, int64_t n, int64_t k, const void* w, const ActP
     if (blocks > n_tiles) blocks = n_tiles;
     if (!plan_ibatch<F>(&p, (int)((n_tiles + blocks - 1) / blocks), warps, (size_t)di->max_smem_optin, &smem)) return kNotSupported;
   } else {
-    // Routed rows: enough rows per pass for most groups (their mean and twice its root), and two thread blocks of eight warps
-    // per SM, so that one computes while the other stages. The kernel deals the tiles of the groups that have rows out
-    // evenly; a grid per group left the SMs to wait for the largest groups, and for blocks of groups without rows.
+    // Routed rows: enough rows per pass for most groups (their mean and twice its root). Two thread blocks of eight warps per
+    // SM, so that one computes while the other stages, where the rows of a whole pass fit half the shared memory; else one
+    // of sixteen, which fits twice as many: staged in chunks, every round of tiles would fetch them again. The kernel
+    // deals the tiles of the groups that have rows out evenly; a grid per group left the SMs to wait for the largest groups,
+    // and for blocks of groups without rows.
     const double mean = (double)n_rows / n_groups;
     int cap = ((int)(mean + 2.0 * sqrt(mean)) + 8) & ~7;
     p.rows_cap = cap < 8 ? 8 : cap > kIbMaxRows ? kIbMaxRows : cap;
-    warps = kIbMaxWarps / 2;
+    const size_t half = ((size_t)di->max_smem_optin + 1024) / 2 - 1024, share = (size_t)3 * 16 * F::kPitch * (kIbMaxWarps / 2);
+    const bool two = p.rows_cap > 32 || (size_t)p.rows_cap * p.nblk * ib_rec(F::kAct) + share + 4096 <= half;
+    if (two) warps = kIbMaxWarps / 2;
     const int64_t all = n_tiles * (n_rows < n_groups ? n_rows : n_groups);
-    if (g_opt.decode_grid == 0) blocks = 2 * di->sm_count;
+    if (g_opt.decode_grid == 0 && two) blocks = 2 * di->sm_count;
     if (blocks > all) blocks = all;
     const int64_t each = (all + blocks - 1) / blocks;
     const int tiles = (int)(each < n_tiles ? each : n_tiles);
-    if (!plan_ibatch<F>(&p, tiles, warps, ((size_t)di->max_smem_optin + 1024) / 2 - 1024, &smem)) {
+    if (!plan_ibatch<F>(&p, tiles, warps, two ? half : (size_t)di->max_smem_optin, &smem)) {
       if (g_opt.decode_grid == 0 && blocks > di->sm_count) blocks = di->sm_count;
       if (!plan_ibatch<F>(&p, tiles, warps, (size_t)di->max_smem_optin, &smem)) return kNotSupported;
     }

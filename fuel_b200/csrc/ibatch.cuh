@@ -507,9 +507,9 @@ using IbQ4_1 = Ib32<4, true>;
 using IbQ5_1 = Ib32<5, true>;
 
 // ------------------------------------------------------------------------------------------------ kernel
-// kGrouped: the rows of many matrices' groups, two blocks of half the warps a SM; else one matrix and one block a SM
+// kGrouped: the rows of many matrices' groups; else one matrix
 template <class F, int MT, bool kGrouped>
-__global__ void __launch_bounds__(32 * (kGrouped || MT > 4 ? kIbMaxWarps / 2 : kIbMaxWarps), kGrouped && MT <= 4 ? 2 : 1) ibatch_kernel(const IbParams p) {
+__global__ void __launch_bounds__(32 * (MT > 4 ? kIbMaxWarps / 2 : kIbMaxWarps), 1) ibatch_kernel(const IbParams p) {
   extern __shared__ __align__(128) uint8_t smem_raw[];
   uint64_t* full = reinterpret_cast<uint64_t*>(smem_raw);  // [2]: an activation buffer's copies have landed
   const uint32_t smem = smem_u32(smem_raw);
@@ -530,28 +530,40 @@ __global__ void __launch_bounds__(32 * (kGrouped || MT > 4 ? kIbMaxWarps / 2 : k
   int grp = 0, m_begin = 0, m_count = p.fixed_rows, t_begin, t_end;
   int base = 0, cost = 0;
   int64_t lo = 0, hi = 0;
+  bool whole = false;  // few groups: every group has blocks of its own, in proportion to its cost, and a block one segment
   if constexpr (!kGrouped) {
     t_begin = (int)((int64_t)n_tiles * blockIdx.x / gridDim.x), t_end = (int)((int64_t)n_tiles * (blockIdx.x + 1) / gridDim.x);
   } else {
-    int total = 0;
-    for (int g = lane; g < p.n_groups; g += 32) total += ib_group_cost(p.offsets[g + 1] - p.offsets[g], p.rows_cap);
+    int total = 0, live = 0;
+    for (int g = lane; g < p.n_groups; g += 32) {
+      const int c = ib_group_cost(p.offsets[g + 1] - p.offsets[g], p.rows_cap);
+      total += c, live += c > 0;
+    }
 #pragma unroll
-    for (int off = 16; off > 0; off >>= 1) total += __shfl_xor_sync(0xffffffffu, total, off);
-    lo = (int64_t)total * n_tiles * blockIdx.x / gridDim.x, hi = (int64_t)total * n_tiles * (blockIdx.x + 1) / gridDim.x;
-    for (;; grp += 32) {  // the group that lo falls into
+    for (int off = 16; off > 0; off >>= 1) total += __shfl_xor_sync(0xffffffffu, total, off), live += __shfl_xor_sync(0xffffffffu, live, off);
+    // from five blocks a group on, rounding to whole blocks costs less than a second segment
+    const int n_blocks = (int)gridDim.x;
+    whole = n_blocks >= 5 * live;
+    lo = (int64_t)total * n_tiles * blockIdx.x / n_blocks, hi = (int64_t)total * n_tiles * (blockIdx.x + 1) / n_blocks;
+    for (;; grp += 32) {  // the group that this block, or lo, falls into
       if (grp >= p.n_groups) return;
-      const int mine = grp + lane < p.n_groups ? ib_group_cost(p.offsets[grp + lane + 1] - p.offsets[grp + lane], p.rows_cap) : 0;
+      int mine = grp + lane < p.n_groups ? ib_group_cost(p.offsets[grp + lane + 1] - p.offsets[grp + lane], p.rows_cap) : 0;
+      if (whole && mine > 0) mine = 1 + (int)((int64_t)(n_blocks - live) * mine / total);
       int upto = mine;
 #pragma unroll
       for (int off = 1; off < 32; off <<= 1) {
         const int v = __shfl_up_sync(0xffffffffu, upto, off);
         if (lane >= off) upto += v;
       }
-      const unsigned past = __ballot_sync(0xffffffffu, (int64_t)(base + upto) * n_tiles > lo);
+      const unsigned past = __ballot_sync(0xffffffffu, whole ? base + upto > (int)blockIdx.x : (int64_t)(base + upto) * n_tiles > lo);
       if (past) {
         const int l = __ffs((int)past) - 1;
         base += __shfl_sync(0xffffffffu, upto - mine, l);
         grp += l;
+        if (whole) {
+          const int part = (int)blockIdx.x - base, parts = __shfl_sync(0xffffffffu, mine, l);
+          t_begin = (int)((int64_t)n_tiles * part / parts), t_end = (int)((int64_t)n_tiles * (part + 1) / parts);
+        }
         break;
       }
       base += __shfl_sync(0xffffffffu, upto, 31);
@@ -562,6 +574,10 @@ __global__ void __launch_bounds__(32 * (kGrouped || MT > 4 ? kIbMaxWarps / 2 : k
     if constexpr (!kGrouped) {
       return t_begin < t_end;
     } else {
+      if (whole) {
+        m_begin = p.offsets[grp], m_count = p.offsets[grp + 1] - m_begin;
+        return t_begin < t_end;
+      }
       for (; grp < p.n_groups && (int64_t)base * n_tiles < hi; ++grp, base += cost) {
         m_begin = p.offsets[grp], m_count = p.offsets[grp + 1] - m_begin;
         cost = ib_group_cost(m_count, p.rows_cap);
@@ -593,36 +609,54 @@ __global__ void __launch_bounds__(32 * (kGrouped || MT > 4 ? kIbMaxWarps / 2 : k
   int64_t gbase;
   int n_pass, rounds;
   int f_tile, f_b, f_stage = 0, f_left;  // next block to fetch
+  constexpr int kPieces = F::kAligned ? F::kBytes256 / 16 : F::kPitch / 16 - 1, kCopies = (16 * kPieces + 31) / 32;
+  // This lane's pieces, lane + 32 i. Formats on 16-byte boundaries: their offsets from the tile's first row, at the block to
+  // fetch, kept for the tile (worked out for every block, they took a tenth of the kernel's instructions), and where they
+  // go: a constant apart where rows are stored without gaps. Others: row | piece << 8.
+  constexpr bool kGapless = F::kAligned && F::kPitch == F::kBytes256;
+  const uint8_t* f_src;
+  uint32_t so[kCopies], rc[kCopies];
+#pragma unroll
+  for (int i = 0; i < kCopies; ++i) {
+    const int q = lane + 32 * i, r = q / kPieces;
+    rc[i] = F::kAligned ? (kGapless ? 16 * q : r * F::kPitch + 16 * (q - r * kPieces)) : r | (q - r * kPieces) << 8;
+  }
+  auto open_tile = [&]() {  // f_tile from block f_b on
+    f_src = p.w + gbase + (int64_t)f_tile * 16 * p.row_bytes + (int64_t)f_b * F::kBytes256;
+    if constexpr (F::kAligned) {
+      const int last = p.n - 1 - f_tile * 16;  // the last tile repeats row n - 1
+#pragma unroll
+      for (int i = 0; i < kCopies; ++i) {
+        const int q = lane + 32 * i, r = q / kPieces;
+        so[i] = (uint32_t)(r < last ? r : last) * (uint32_t)p.row_bytes + 16u * (uint32_t)(q - r * kPieces);
+      }
+    }
+  };
   auto start_stream = [&]() {  // for the segment's tiles slot, slot + tg, ...
     gbase = kGrouped ? (int64_t)grp * p.group_bytes : 0;
     n_pass = (m_count + p.rows_cap - 1) / p.rows_cap;
     rounds = (t_end - t_begin + p.tg - 1) / p.tg;
     const int mine = has_slot && t_end - t_begin > slot ? (t_end - t_begin - slot + p.tg - 1) / p.tg : 0;
     f_tile = t_begin + slot, f_b = b_begin, f_left = mine * nb * n_pass;
+    open_tile();
   };
-  constexpr int kPieces = F::kAligned ? F::kBytes256 / 16 : F::kPitch / 16 - 1, kCopies = (16 * kPieces + 31) / 32;
-  int rc[kCopies];  // this lane's pieces: row | piece << 8, or -1
-#pragma unroll
-  for (int i = 0; i < kCopies; ++i) {
-    const int q = lane + 32 * i, r = q / kPieces;
-    rc[i] = q < 16 * kPieces ? r | (q - r * kPieces) << 8 : -1;
-  }
   auto fetch = [&]() {  // one block of this warp's tile into the next stage; always one commit group
     if (f_left > 0) {
       --f_left;
       const uint32_t dst = wst + (uint32_t)f_stage * stage_bytes;
-      const int64_t o = gbase + (int64_t)(f_tile * 16) * p.row_bytes + (int64_t)f_b * F::kBytes256;  // offset of row 0
-      const uint8_t* src = p.w + o;
-      if (f_tile + 1 < n_tiles || F::kAligned) {
-        const int last = p.n - 1 - f_tile * 16;  // the last tile repeats row n - 1
+      if constexpr (F::kAligned) {
+#pragma unroll
+        for (int i = 0; i < kCopies; ++i)
+          if (32 * i + 32 <= 16 * kPieces || lane + 32 * i < 16 * kPieces) ib_cp16(dst + rc[i], f_src + so[i], 16u);
+      } else if (f_tile + 1 < n_tiles) {
 #pragma unroll
         for (int i = 0; i < kCopies; ++i) {
-          if (rc[i] >= 0) {
+          if (32 * i + 32 <= 16 * kPieces || lane + 32 * i < 16 * kPieces) {
             const int r = rc[i] & 255, c = rc[i] >> 8;
-            const int ro = (r < last ? r : last) * p.row_bytes;
-            const int skew = F::kAligned ? 0 : ((int)o + ro) & 15;
-            if (F::kAligned || 16 * c < skew + F::kBytes256)
-              ib_cp16(dst + (uint32_t)(r * F::kPitch + 16 * c), src + (ro - skew + 16 * c), 16u);
+            const uint8_t* row = f_src + r * p.row_bytes;
+            const int skew = (int)(reinterpret_cast<uintptr_t>(row) & 15);  // the matrix starts on a 16-byte boundary
+            if (16 * (kPieces - 1) < F::kBytes256 || 16 * c < skew + F::kBytes256)
+              ib_cp16(dst + (uint32_t)(r * F::kPitch + 16 * c), row - skew + 16 * c, 16u);
           }
         }
       } else {  // the matrix may end inside a 16-byte piece: read only what it has
@@ -636,10 +670,12 @@ __global__ void __launch_bounds__(32 * (kGrouped || MT > 4 ? kIbMaxWarps / 2 : k
         }
       }
       if (++f_stage == p.stages) f_stage = 0;
+      f_src += F::kBytes256;
       if (++f_b == b_end) {
         f_b = b_begin;
         f_tile += p.tg;
         if (f_tile >= t_end) f_tile = t_begin + slot;  // next pass over the rows
+        open_tile();
       }
     }
     ib_commit();
@@ -814,7 +850,7 @@ __global__ void __launch_bounds__(32 * (kGrouped || MT > 4 ? kIbMaxWarps / 2 : k
         }
       }
     }
-    if constexpr (!kGrouped) break;
+    if (!kGrouped || whole) break;
     ++grp, base += cost;
     if (!segment()) break;
   }
