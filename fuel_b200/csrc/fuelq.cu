@@ -650,6 +650,7 @@ int32_t ibatch_fmt(int n_groups, int64_t n, int64_t k, const void* w, const ActP
   int64_t blocks = g_opt.decode_grid > 0 ? g_opt.decode_grid : di->sm_count;
   if constexpr (!kGrouped) {
     p.rows_cap = n_rows >= kIbMaxRows ? kIbMaxRows : (int)((n_rows + 7) & ~7ll);
+    if (p.rows_cap > 32) p.rows_cap = (p.rows_cap + 15) & ~15;
     if (p.rows_cap > 32) warps = kIbMaxWarps / 2;  // twice the registers a thread
     if (blocks > n_tiles) blocks = n_tiles;
     if (!plan_ibatch<F>(&p, (int)((n_tiles + blocks - 1) / blocks), warps, (size_t)di->max_smem_optin, &smem)) return kNotSupported;
@@ -679,7 +680,9 @@ int32_t ibatch_fmt(int n_groups, int64_t n, int64_t k, const void* w, const ActP
   cudaError_t e;
   if (p.rows_cap <= 8) e = launch_ibatch<F, 1, kGrouped>(p, grid, warps, smem, stream);
   else if (p.rows_cap <= 16) e = launch_ibatch<F, 2, kGrouped>(p, grid, warps, smem, stream);
+  else if (!kGrouped && p.rows_cap <= 24) e = launch_ibatch<F, kGrouped ? 4 : 3, kGrouped>(p, grid, warps, smem, stream);
   else if (p.rows_cap <= 32) e = launch_ibatch<F, 4, kGrouped>(p, grid, warps, smem, stream);
+  else if (!kGrouped && p.rows_cap <= 48) e = launch_ibatch<F, kGrouped ? 8 : 6, kGrouped>(p, grid, warps, smem, stream);
   else e = launch_ibatch<F, 8, kGrouped>(p, grid, warps, smem, stream);
   return e == cudaSuccess ? kOk : kLaunchFailure;
 }
@@ -826,8 +829,8 @@ bool prefill_available(int type, int64_t m, int64_t n, int64_t k) {
   (void)n;
   int64_t max_m = g_opt.decode_max_m;
   if (max_m == 0) {
-    // The library's choice: 16 rows; 64 where the integer tensor-core kernel applies (16 rows per pass over the weights,
-    // the later passes from L2) - still faster there than the bf16 GEMM, and the reference's own arithmetic.
+    // The library's choice: 16 rows; 64 where the integer tensor-core kernel applies (one pass over
+    // the weights) - still faster there than the bf16 GEMM, and the reference's own arithmetic.
     max_m = 16;
     if ((prefill_native_type(type) || type == kQ5K) && g_opt.decode_kernel == 0 && g_opt.moe_kernel == 0 && k % 256 == 0) max_m = 64;
   }

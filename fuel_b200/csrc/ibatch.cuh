@@ -148,6 +148,17 @@ struct IbCtx {
   int lane, gid, tig, nt;
 };
 
+// The activation tiles of a step, in parts that run together: with a branch around each tile, none of one tile's loads and
+// products can be issued under the latency of another's (Q4_K 11008 x 4096, 48 rows: 45 us, with parts 36); with all of eight,
+// or three of the sixteen-group formats at the sixteen-warp form's 128 registers, the registers spill (64 rows: 51 and 77 us).
+// kSingly: a branch around each tile all the same (the grouped form for up to 64 rows, where any number of tiles occurs).
+__host__ __device__ constexpr int ib_part(int nt, bool singly, int small, int large) {
+  return singly ? 1 : nt <= 2 ? nt : nt <= 4 ? (small < nt ? small : nt) : nt <= 6 ? nt : large;
+}
+#define FQ_IB_TILES(SMALL, LARGE)                                                                                  \
+  _Pragma("unroll") for (int mq = 0; mq < NT; mq += ib_part(NT, kSingly, SMALL, LARGE)) if (mq == 0 || mq < cx.nt) \
+      _Pragma("unroll") for (int mt = mq; mt < NT && mt < mq + ib_part(NT, kSingly, SMALL, LARGE); ++mt)
+
 // Quant fragments of activation tile mt for 64 elements from element 64 * g: b[0..1] the first 32, b[2..3] the second
 template <int kRec = kActRecord>
 __device__ __forceinline__ void ib_b64(const IbCtx& cx, int mt, int g, uint32_t (&b)[4]) {
@@ -175,7 +186,7 @@ struct IbQ45K {
   static constexpr int kBytes256 = kFive ? 176 : 144, kPitch = kBytes256;  // 144 and 176 both spread eight rows over the banks
   static constexpr bool kAligned = true;
   static constexpr IbAct kAct = kIbQ8K;
-  template <int MT>
+  template <int NT, bool kSingly, int MT>
   __device__ __forceinline__ static void block(const IbCtx& cx, float (&facc)[MT][4]) {
     const uint4 h0 = lds128(cx.r0), h1 = lds128(cx.r1);
     // eight 6-bit scales / mins per row as bytes of two words (get_scale_min_k4, fuel-quantized/src/utils.rs:50-60)
@@ -192,7 +203,7 @@ struct IbQ45K {
     }
     uint32_t hq[4];
     if constexpr (kFive) ldmatrix_x4(hq, cx.lm + 16u);
-    int S[MT][4];
+    int S[NT][4];
 #pragma unroll
     for (int g = 0; g < 4; ++g) {  // 64 elements: low nibbles = sub-block 2g, high nibbles = 2g + 1
       uint32_t r[4], lo[4], hi[4];
@@ -207,28 +218,24 @@ struct IbQ45K {
       }
       const int s0l = ib_byte(sc0[g >> 1], 2 * (g & 1)), s0h = ib_byte(sc0[g >> 1], 2 * (g & 1) + 1);
       const int s1l = ib_byte(sc1[g >> 1], 2 * (g & 1)), s1h = ib_byte(sc1[g >> 1], 2 * (g & 1) + 1);
-#pragma unroll
-      for (int mt = 0; mt < MT; ++mt) {
-        if (mt < cx.nt) {
-          uint32_t b[4];
-          ib_b64(cx, mt, g, b);
-          int cl[4], ch[4];
-          mma_u8_k32<true>(cl, lo, b[0], b[1]);
-          mma_u8_k32<true>(ch, hi, b[2], b[3]);
-          int (&T)[4] = S[mt];
-          if (g == 0) {
-            T[0] = cl[0] * s0l + ch[0] * s0h, T[1] = cl[1] * s0l + ch[1] * s0h;
-            T[2] = cl[2] * s1l + ch[2] * s1h, T[3] = cl[3] * s1l + ch[3] * s1h;
-          } else {
-            T[0] += cl[0] * s0l + ch[0] * s0h, T[1] += cl[1] * s0l + ch[1] * s0h;
-            T[2] += cl[2] * s1l + ch[2] * s1h, T[3] += cl[3] * s1l + ch[3] * s1h;
-          }
+      FQ_IB_TILES(4, 4) {
+        uint32_t b[4];
+        ib_b64(cx, mt, g, b);
+        int cl[4], ch[4];
+        mma_u8_k32<true>(cl, lo, b[0], b[1]);
+        mma_u8_k32<true>(ch, hi, b[2], b[3]);
+        int (&T)[4] = S[mt];
+        if (g == 0) {
+          T[0] = cl[0] * s0l + ch[0] * s0h, T[1] = cl[1] * s0l + ch[1] * s0h;
+          T[2] = cl[2] * s1l + ch[2] * s1h, T[3] = cl[3] * s1l + ch[3] * s1h;
+        } else {
+          T[0] += cl[0] * s0l + ch[0] * s0h, T[1] += cl[1] * s0l + ch[1] * s0h;
+          T[2] += cl[2] * s1l + ch[2] * s1h, T[3] += cl[3] * s1l + ch[3] * s1h;
         }
       }
     }
-#pragma unroll
-    for (int mt = 0; mt < MT; ++mt)
-      if (mt < cx.nt) ib_finish_min<MT>(cx, mt, am, S[mt], d0, dm0, d1, dm1, facc);
+    FQ_IB_TILES(4, 4)
+      ib_finish_min(cx, mt, am, S[mt], d0, dm0, d1, dm1, facc);
   }
 };
 using IbQ4K = IbQ45K<false>;
@@ -237,39 +244,33 @@ using IbQ5K = IbQ45K<true>;
 // ------------------------------------------------------------------------------------------------ Q6_K, Q3_K
 // Sixteen groups of 16 elements, each with a signed scale (bytes of sc0 / sc1 for rows gid / gid + 8): step g takes groups
 // 4g .. 4g + 3, A[i] = the left-justified values of group 4g + i
-template <int MT>
-__device__ __forceinline__ void ib_groups16_step(const IbCtx& cx, int g, const uint32_t (&A)[4][2], uint32_t sc0, uint32_t sc1, int (&S)[MT][4]) {
+template <int NT, bool kSingly>
+__device__ __forceinline__ void ib_groups16_step(const IbCtx& cx, int g, const uint32_t (&A)[4][2], uint32_t sc0, uint32_t sc1, int (&S)[NT][4]) {
   int s0[4], s1[4];
 #pragma unroll
   for (int i = 0; i < 4; ++i) s0[i] = ib_sbyte(sc0, i), s1[i] = ib_sbyte(sc1, i);
+  FQ_IB_TILES(2, 4) {
+    uint32_t b[4];
+    ib_b64(cx, mt, g, b);
+    int (&T)[4] = S[mt];
 #pragma unroll
-  for (int mt = 0; mt < MT; ++mt) {
-    if (mt < cx.nt) {
-      uint32_t b[4];
-      ib_b64(cx, mt, g, b);
-      int (&T)[4] = S[mt];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        int c[4];
-        mma_s8_k16(c, A[i][0], A[i][1], b[i]);
-        if (g == 0 && i == 0) T[0] = c[0] * s0[i], T[1] = c[1] * s0[i], T[2] = c[2] * s1[i], T[3] = c[3] * s1[i];
-        else T[0] += c[0] * s0[i], T[1] += c[1] * s0[i], T[2] += c[2] * s1[i], T[3] += c[3] * s1[i];
-      }
+    for (int i = 0; i < 4; ++i) {
+      int c[4];
+      mma_s8_k16(c, A[i][0], A[i][1], b[i]);
+      if (g == 0 && i == 0) T[0] = c[0] * s0[i], T[1] = c[1] * s0[i], T[2] = c[2] * s1[i], T[3] = c[3] * s1[i];
+      else T[0] += c[0] * s0[i], T[1] += c[1] * s0[i], T[2] += c[2] * s1[i], T[3] += c[3] * s1[i];
     }
   }
 }
-template <int MT>
-__device__ __forceinline__ void ib_groups16_finish(const IbCtx& cx, const int (&S)[MT][4], float d0, float d1, float (&facc)[MT][4]) {
-#pragma unroll
-  for (int mt = 0; mt < MT; ++mt) {
-    if (mt < cx.nt) {
-      const uint32_t da = cx.act + (uint32_t)(8 * mt + 2 * cx.tig) * kActRecord + kActRecD;
-      const float ya = __uint_as_float(lds32(da)), yb = __uint_as_float(lds32(da + kActRecord));
-      facc[mt][0] += (d0 * ya) * (float)S[mt][0];
-      facc[mt][1] += (d0 * yb) * (float)S[mt][1];
-      facc[mt][2] += (d1 * ya) * (float)S[mt][2];
-      facc[mt][3] += (d1 * yb) * (float)S[mt][3];
-    }
+template <int NT, bool kSingly, int MT>
+__device__ __forceinline__ void ib_groups16_finish(const IbCtx& cx, const int (&S)[NT][4], float d0, float d1, float (&facc)[MT][4]) {
+  FQ_IB_TILES(2, 4) {
+    const uint32_t da = cx.act + (uint32_t)(8 * mt + 2 * cx.tig) * kActRecord + kActRecD;
+    const float ya = __uint_as_float(lds32(da)), yb = __uint_as_float(lds32(da + kActRecord));
+    facc[mt][0] += (d0 * ya) * (float)S[mt][0];
+    facc[mt][1] += (d0 * yb) * (float)S[mt][1];
+    facc[mt][2] += (d1 * ya) * (float)S[mt][2];
+    facc[mt][3] += (d1 * yb) * (float)S[mt][3];
   }
 }
 
@@ -277,9 +278,9 @@ struct IbQ6K {
   static constexpr int kBytes256 = 210, kPitch = 240;  // fetched as 14 16-byte pieces (skew 0..14)
   static constexpr bool kAligned = false;
   static constexpr IbAct kAct = kIbQ8K;
-  template <int MT>
+  template <int NT, bool kSingly, int MT>
   __device__ __forceinline__ static void block(const IbCtx& cx, float (&facc)[MT][4]) {
-    int S[MT][4];
+    int S[NT][4];
     // 4 * (q - 32) of quadrant q of half h: elements 128 h + 32 q + l (k_quants.rs:2170-2185), l = 16 s + 4 tig .. + 3
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
@@ -305,11 +306,11 @@ struct IbQ6K {
             A[2 + s][r] = ((b & 0x3c3c3c3cu) ^ 0x80808080u) ^ (hb & 0xc0c0c0c0u);
           }
         const int g = 2 * h + u;
-        ib_groups16_step<MT>(cx, g, A, lds_u32_2b_addr(cx.r0 + 192u + 4u * g), lds_u32_2b_addr(cx.r1 + 192u + 4u * g), S);
+        ib_groups16_step<NT, kSingly>(cx, g, A, lds_u32_2b_addr(cx.r0 + 192u + 4u * g), lds_u32_2b_addr(cx.r1 + 192u + 4u * g), S);
       }
     }
     const float d0 = 0.25f * h2f_bits(lds_u16_addr(cx.r0 + 208u)), d1 = 0.25f * h2f_bits(lds_u16_addr(cx.r1 + 208u));
-    ib_groups16_finish<MT>(cx, S, d0, d1, facc);
+    ib_groups16_finish<NT, kSingly>(cx, S, d0, d1, facc);
   }
 };
 
@@ -326,12 +327,12 @@ struct IbQ3K {
 #pragma unroll
     for (int i = 0; i < 4; ++i) sc[i] = ((sc[i] | 0x80808080u) - 0x20202020u) ^ 0x80808080u;
   }
-  template <int MT>
+  template <int NT, bool kSingly, int MT>
   __device__ __forceinline__ static void block(const IbCtx& cx, float (&facc)[MT][4]) {
     uint32_t sc0[4], sc1[4], hm[2][2];  // hm: [s][row]
     scales(cx.r0, sc0);
     scales(cx.r1, sc1);
-    int S[MT][4];
+    int S[NT][4];
 #pragma unroll
     for (int s = 0; s < 2; ++s)
 #pragma unroll
@@ -356,11 +357,11 @@ struct IbQ3K {
               const int j = 2 * u + jj;
               A[2 * jj + s][r] = (((q[s][r] >> (2 * j)) & 0x03030303u) << 5) ^ ((((hm[s][r] >> (4 * c + j)) & 0x01010101u) << 7) ^ 0x80808080u);
             }
-        ib_groups16_step<MT>(cx, 2 * c + u, A, sc0[2 * c + u], sc1[2 * c + u], S);
+        ib_groups16_step<NT, kSingly>(cx, 2 * c + u, A, sc0[2 * c + u], sc1[2 * c + u], S);
       }
     }
     const float d0 = 0.03125f * h2f_bits(lds_u16_addr(cx.r0 + 108u)), d1 = 0.03125f * h2f_bits(lds_u16_addr(cx.r1 + 108u));
-    ib_groups16_finish<MT>(cx, S, d0, d1, facc);
+    ib_groups16_finish<NT, kSingly>(cx, S, d0, d1, facc);
   }
 };
 
@@ -369,7 +370,7 @@ struct IbQ2K {
   static constexpr int kBytes256 = 84, kPitch = 112;  // fetched as six or seven pieces (skew 0, 4, 8, 12)
   static constexpr bool kAligned = false;
   static constexpr IbAct kAct = kIbQ8K;
-  template <int MT>
+  template <int NT, bool kSingly, int MT>
   __device__ __forceinline__ static void block(const IbCtx& cx, float (&facc)[MT][4]) {
     uint32_t am[4], sw[2][4];
 #pragma unroll
@@ -380,7 +381,7 @@ struct IbQ2K {
       const uint32_t ma = lds_u16_addr(row + 2u * cx.tig), mb = lds_u16_addr(row + 8u + 2u * cx.tig);
       am[r] = ib_h2((int)((ma >> 4) & 0xfu), (int)(ma >> 12)), am[2 + r] = ib_h2((int)((mb >> 4) & 0xfu), (int)(mb >> 12));
     }
-    int S[MT][4];
+    int S[NT][4];
 #pragma unroll
     for (int c = 0; c < 2; ++c) {
       uint32_t q[2][2];  // [s][row]
@@ -400,23 +401,19 @@ struct IbQ2K {
               const int j = 2 * u + jj, gr = 8 * c + 2 * j + s;
               A[jj][2 * s + r] = ((q[s][r] >> (2 * j)) & 0x03030303u) * (uint32_t)(ib_byte(sw[r][gr >> 2], gr & 3) & 0xf);  // at most 45 a byte
             }
-#pragma unroll
-        for (int mt = 0; mt < MT; ++mt) {
-          if (mt < cx.nt) {
-            uint32_t b[4];
-            ib_b64(cx, mt, 2 * c + u, b);
-            if (c == 0 && u == 0) mma_u8_k32<true>(S[mt], A[0], b[0], b[1]);
-            else mma_u8_k32<false>(S[mt], A[0], b[0], b[1]);
-            mma_u8_k32<false>(S[mt], A[1], b[2], b[3]);
-          }
+        FQ_IB_TILES(4, 4) {
+          uint32_t b[4];
+          ib_b64(cx, mt, 2 * c + u, b);
+          if (c == 0 && u == 0) mma_u8_k32<true>(S[mt], A[0], b[0], b[1]);
+          else mma_u8_k32<false>(S[mt], A[0], b[0], b[1]);
+          mma_u8_k32<false>(S[mt], A[1], b[2], b[3]);
         }
       }
     }
     const uint32_t dd0 = lds32(cx.r0 + 80u), dd1 = lds32(cx.r1 + 80u);
     const float d0 = h2f_bits(dd0 & 0xffffu), dm0 = h2f_bits(dd0 >> 16), d1 = h2f_bits(dd1 & 0xffffu), dm1 = h2f_bits(dd1 >> 16);
-#pragma unroll
-    for (int mt = 0; mt < MT; ++mt)
-      if (mt < cx.nt) ib_finish_min<MT>(cx, mt, am, S[mt], d0, dm0, d1, dm1, facc);
+    FQ_IB_TILES(4, 4)
+      ib_finish_min(cx, mt, am, S[mt], d0, dm0, d1, dm1, facc);
   }
 };
 
@@ -459,7 +456,7 @@ struct Ib32 {
       }
     }
   }
-  template <int MT>
+  template <int NT, bool kSingly, int MT>
   __device__ __forceinline__ static void block(const IbCtx& cx, float (&facc)[MT][4]) {
 #pragma unroll
     for (int g = 0; g < 4; ++g) {  // two 32-element blocks at a time
@@ -470,30 +467,27 @@ struct Ib32 {
         row_block(cx.r0 + (uint32_t)(kBlk * (2 * g + h)), cx.tig, A[h][0], A[h][2], d0[h], m0[h]);
         row_block(cx.r1 + (uint32_t)(kBlk * (2 * g + h)), cx.tig, A[h][1], A[h][3], d1[h], m1[h]);
       }
+      FQ_IB_TILES(4, 4) {
+        uint32_t b[4];
+        constexpr int kRec = ib_rec(kAct);
+        ib_b64<kRec>(cx, mt, g, b);
+        const uint32_t da = cx.act + (uint32_t)(8 * mt + 2 * cx.tig) * kRec + kActRecAux + 8u * g;
+        const uint2 ya = lds64(da), yb = lds64(da + kRec);
+        uint2 sa = make_uint2(0, 0), sb = sa;
+        if constexpr (kMin) sa = lds64(da + 32u), sb = lds64(da + 32u + kRec);
 #pragma unroll
-      for (int mt = 0; mt < MT; ++mt) {
-        if (mt < cx.nt) {
-          uint32_t b[4];
-          constexpr int kRec = ib_rec(kAct);
-          ib_b64<kRec>(cx, mt, g, b);
-          const uint32_t da = cx.act + (uint32_t)(8 * mt + 2 * cx.tig) * kRec + kActRecAux + 8u * g;
-          const uint2 ya = lds64(da), yb = lds64(da + kRec);
-          uint2 sa = make_uint2(0, 0), sb = sa;
-          if constexpr (kMin) sa = lds64(da + 32u), sb = lds64(da + 32u + kRec);
-#pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            int c[4];
-            if constexpr (kMin) mma_u8_k32<true>(c, A[h], b[2 * h], b[2 * h + 1]);
-            else mma_s8_k32<true>(c, A[h], b[2 * h], b[2 * h + 1]);
-            const float fa = __uint_as_float(h ? ya.y : ya.x), fb = __uint_as_float(h ? yb.y : yb.x);
-            facc[mt][0] += (d0[h] * fa) * (float)c[0];
-            facc[mt][1] += (d0[h] * fb) * (float)c[1];
-            facc[mt][2] += (d1[h] * fa) * (float)c[2];
-            facc[mt][3] += (d1[h] * fb) * (float)c[3];
-            if constexpr (kMin) {
-              const float ga = __uint_as_float(h ? sa.y : sa.x), gb = __uint_as_float(h ? sb.y : sb.x);
-              facc[mt][0] += m0[h] * ga, facc[mt][1] += m0[h] * gb, facc[mt][2] += m1[h] * ga, facc[mt][3] += m1[h] * gb;
-            }
+        for (int h = 0; h < 2; ++h) {
+          int c[4];
+          if constexpr (kMin) mma_u8_k32<true>(c, A[h], b[2 * h], b[2 * h + 1]);
+          else mma_s8_k32<true>(c, A[h], b[2 * h], b[2 * h + 1]);
+          const float fa = __uint_as_float(h ? ya.y : ya.x), fb = __uint_as_float(h ? yb.y : yb.x);
+          facc[mt][0] += (d0[h] * fa) * (float)c[0];
+          facc[mt][1] += (d0[h] * fb) * (float)c[1];
+          facc[mt][2] += (d1[h] * fa) * (float)c[2];
+          facc[mt][3] += (d1[h] * fb) * (float)c[3];
+          if constexpr (kMin) {
+            const float ga = __uint_as_float(h ? sa.y : sa.x), gb = __uint_as_float(h ? sb.y : sb.x);
+            facc[mt][0] += m0[h] * ga, facc[mt][1] += m0[h] * gb, facc[mt][2] += m1[h] * ga, facc[mt][3] += m1[h] * gb;
           }
         }
       }
@@ -507,6 +501,18 @@ using IbQ4_1 = Ib32<4, true>;
 using IbQ5_1 = Ib32<5, true>;
 
 // ------------------------------------------------------------------------------------------------ kernel
+// The step's block times the first cx.nt tiles, whose number is a constant in the arithmetic
+template <class F, int NT, int MT>
+__device__ __forceinline__ void ib_block(const IbCtx& cx, float (&facc)[MT][4]) {
+  if constexpr (NT < MT) {
+    if (cx.nt > NT) {
+      ib_block<F, NT + 1>(cx, facc);
+      return;
+    }
+  }
+  F::template block<NT, false>(cx, facc);
+}
+
 // kGrouped: the rows of many matrices' groups; else one matrix
 template <class F, int MT, bool kGrouped>
 __global__ void __launch_bounds__(32 * (MT > 4 ? kIbMaxWarps / 2 : kIbMaxWarps), 1) ibatch_kernel(const IbParams p) {
@@ -741,7 +747,7 @@ __global__ void __launch_bounds__(32 * (MT > 4 ? kIbMaxWarps / 2 : kIbMaxWarps),
     for (int i = 0; i < p.stages - 1; ++i) fetch();
     if (first && early) pdl_wait();
     // the plan's chunks are for rows_cap rows: fewer need fewer chunks
-    slot_bytes = (n_pass == 1 ? (m_count + 7) & ~7 : p.rows_cap) * kRec;
+    slot_bytes = (kGrouped && n_pass == 1 ? (m_count + 7) & ~7 : p.rows_cap) * kRec;
     bpc = p.bpc, n_chunks = p.n_chunks;
     if (kGrouped && n_chunks > 1) {
       const int share = p.share_q + (p.share_rem > 0);
@@ -793,7 +799,8 @@ __global__ void __launch_bounds__(32 * (MT > 4 ? kIbMaxWarps / 2 : kIbMaxWarps),
             cx.r1 = st + (uint32_t)((cx.gid + 8) * F::kPitch) + k1;
             cx.lm = st + (uint32_t)(((lane & 7) + (lane & 8)) * F::kPitch) + 16u * (lane >> 4);
             cx.act = abase + (uint32_t)((kpart * bpc + j) * slot_bytes);
-            F::template block<MT>(cx, facc);
+            if constexpr (kGrouped && MT > 4) F::template block<MT, true>(cx, facc);
+            else ib_block<F, kGrouped ? 1 : MT>(cx, facc);
             __syncwarp();  // every lane has read the stage before any lane refills it
           }
           if (more) {
@@ -827,7 +834,7 @@ __global__ void __launch_bounds__(32 * (MT > 4 ? kIbMaxWarps / 2 : kIbMaxWarps),
 #pragma unroll
                 for (int q = 0; q < (MT > 1 ? 2 : 1); ++q)
 #pragma unroll
-                  for (int i = 0; i < 4; ++i) part[warp * kW + (q * 4 + i) * 32 + lane] = facc[m2 + q][i];
+                  for (int i = 0; i < 4; ++i) if (m2 + q < MT) part[warp * kW + (q * 4 + i) * 32 + lane] = facc[m2 + q][i];
               }
               __syncthreads();
               const int tiles_here = t_end - (t_begin + round * p.tg) < p.tg ? t_end - (t_begin + round * p.tg) : p.tg;
@@ -856,4 +863,5 @@ __global__ void __launch_bounds__(32 * (MT > 4 ? kIbMaxWarps / 2 : kIbMaxWarps),
   }
 }
 
+#undef FQ_IB_TILES
 }  // namespace fq

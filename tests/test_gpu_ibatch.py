@@ -33,3 +33,38 @@ def test_batch_edges_match_the_oracle(oracle, name):
     finally:
         _lib.lib.fuelq_set_option(_lib.OPT_DECODE_MAX_M, 0)
     assert ops.device_error() == 0
+
+
+@pytest.mark.parametrize("name", ("Q4K", "Q6K"))
+@pytest.mark.parametrize("counts,n,k", [
+    ([0, 3, 0, 0, 1, 0, 0, 9] + [0] * 56, 293, 768),          # few groups: blocks of their own
+    ([1] * 70 + [0] * 5 + [40] + [2] * 52, 37, 512),          # many: blocks that span several, one group in several passes
+    ([17, 0, 33, 24, 8, 130, 1, 16] * 5, 165, 2304),          # up to 64 rows a pass, and more
+    ([26, 31, 12, 0, 25, 18, 32, 20] * 16, 85, 2048),         # some twenty rows each: sixteen warps a block
+])
+def test_groups_match_the_oracle(oracle, name, counts, n, k):
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from fuel_b200 import GgmlDType as T, _lib, ops
+    from test_gpu_kernels import assert_matmul_close
+    t, ot, L = getattr(T, name), getattr(oracle, name), _lib.lib
+    g = np.random.Generator(np.random.PCG64(5))
+    e, rows = len(counts), sum(counts)
+    wb = oracle.quantize(ot, g.standard_normal((e * n, k), dtype=np.float32) * np.float32(0.02))
+    x = g.standard_normal((rows, k), dtype=np.float32)
+    off = np.concatenate([[0], np.cumsum(counts)]).astype(np.int32)
+    order = g.permutation(rows).astype(np.int32)               # where each row's result goes
+    xd, wd, od, rd = (torch.from_numpy(a).cuda() for a in (x, wb, off, order))
+    ids = torch.arange(rows, dtype=torch.int32, device="cuda")
+    packed = torch.empty(L.fuelq_act_packed_bytes(int(T.Q4K), rows, k), dtype=torch.uint8, device="cuda")
+    y = torch.full((rows, n), float("nan"), device="cuda")
+    st = torch.cuda.current_stream().cuda_stream
+    _lib.check(L.fuelq_moe_quantize_rows(xd.data_ptr(), k, ids.data_ptr(), 1, rows, packed.data_ptr(), packed.numel(), st), "quantize")
+    _lib.check(L.fuelq_moe_qmatmul(int(t), e, n, k, wd.data_ptr(), packed.data_ptr(), rows, od.data_ptr(), rd.data_ptr(), y.data_ptr(), st), "qmatmul")
+    got = y.cpu().numpy()[order]
+    per = wb.size // e
+    for i, c in enumerate(counts):
+        if c:
+            r = slice(off[i], off[i] + c)
+            assert_matmul_close(got[r], oracle.matmul(ot, x[r], wb.reshape(-1)[i * per:(i + 1) * per], n), (name, i, c))
+    assert ops.device_error() == 0
