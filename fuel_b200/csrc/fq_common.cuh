@@ -216,7 +216,7 @@ __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepc
 // of the next matrix overlaps the current one's arithmetic and the dependency bubble between
 // kernels. It ends with pdl_wait() so that kernels ordered after it still wait, transitively,
 // for everything before it.
-__global__ void __launch_bounds__(32) prefetch_l2_kernel(const uint8_t* __restrict__ w, long long bytes) {
+static __global__ void __launch_bounds__(32) prefetch_l2_kernel(const uint8_t* __restrict__ w, long long bytes) {
   pdl_launch_dependents();
   const long long chunk = 4096;
   const long long n_chunks = (bytes & ~15ll) / chunk;
@@ -235,7 +235,7 @@ __global__ void __launch_bounds__(32) prefetch_l2_kernel(const uint8_t* __restri
 
 // n f32 words from device memory to a device-mapped host buffer (or any other place), 16 bytes per thread where
 // both addresses allow it: the write-back of a small result without a copy-engine hand-off.
-__global__ void __launch_bounds__(256) copy_out_f32_kernel(const float* __restrict__ src, float* __restrict__ dst, long long n,
+static __global__ void __launch_bounds__(256) copy_out_f32_kernel(const float* __restrict__ src, float* __restrict__ dst, long long n,
                                                            int vec) {
   pdl_launch_dependents();
   pdl_wait();
@@ -268,7 +268,7 @@ __device__ __forceinline__ uint32_t lds_u16(const uint8_t* p) {
 __device__ __forceinline__ float h2f_bits(uint32_t h) { return __half2float(__ushort_as_half((unsigned short)h)); }
 
 // defined once: the library is a single translation unit
-__device__ int g_fq_dev_error = 0;
+static __device__ int g_fq_dev_error = 0;  // one in each of the library's translation units
 __device__ __forceinline__ void record_dev_error(int code) { atomicCAS(&g_fq_dev_error, 0, code); }
 
 #endif  // __CUDACC__

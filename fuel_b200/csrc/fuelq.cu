@@ -13,6 +13,7 @@
 #include "dequantize.cuh"
 #include "fq_common.cuh"
 #include "ibatch.cuh"
+#include "launch.cuh"
 #include "llama_glue.cuh"
 #include "moe.cuh"
 #include "plain_gemm.cuh"
@@ -70,31 +71,6 @@ inline bool aligned(const void* p, size_t a) { return (reinterpret_cast<uintptr_
 bool supported_weight(int t) {
   return t == kQ4_0 || t == kQ4_1 || t == kQ5_0 || t == kQ5_1 || t == kQ8_0 || t == kQ2K || t == kQ3K || t == kQ4K || t == kQ5K ||
          t == kQ6K;
-}
-
-// Every kernel goes out with the programmatic-dependent-launch attribute: all of them call griddepcontrol.wait before they
-// touch memory an earlier kernel of the stream may have written, so the attribute changes when a kernel's blocks are put on
-// the SMs, never what they see. What FUELQ_OPT_PDL adds is the caller's promise that WEIGHTS are not written by the stream's
-// preceding work, which lets a call's first kernel stream them before that wait (`early_w` of the mat-vec kernels; the later
-// kernels of a call always may: its first kernel lets them start only after its own wait, see quantize_q8k_kernel's
-// `late_trigger`).
-template <typename... KArgs, typename... Args>
-cudaError_t launch_if(bool dependent, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = grid;
-  cfg.blockDim = block;
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = dependent ? 1 : 0;
-  return cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...);
-}
-template <typename... KArgs, typename... Args>
-cudaError_t launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args) {
-  return launch_if(true, kernel, grid, block, smem, stream, args...);
 }
 
 // ------------------------------------------------------------------ activation quantization
@@ -569,23 +545,6 @@ int32_t prefetch_impl(const void* w, int64_t bytes, cudaStream_t stream) {
 }
 
 // ---- a few to a few dozen rows on the integer tensor cores (ibatch.cuh): every format, k a multiple of 256
-template <class F, int MT, bool kGrouped>
-cudaError_t launch_ibatch(const IbParams& p, dim3 grid, int warps, size_t smem, cudaStream_t stream) {
-  static bool attr_set[64] = {};
-  auto kern = ibatch_kernel<F, MT, kGrouped>;
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
-  if (!attr_set[dev]) {
-    DeviceInfo* di;
-    if (!device_info(&di)) return cudaErrorInvalidDevice;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, di->max_smem_optin);
-    if (e != cudaSuccess) return e;
-    attr_set[dev] = true;
-  }
-  return launch(kern, grid, dim3(32 * warps), smem, stream, p);
-}
-
 // Shared-memory plan for `tiles` 16-row tiles per thread block of `warps` warps. The split of the warps over tiles and k is
 // the one with the fewest steps (one block of one tile each) on a warp's critical path.
 template <class F>
@@ -625,7 +584,7 @@ bool plan_ibatch(IbParams* p, int tiles, int warps, size_t budget, size_t* smem)
 }
 
 template <class F, bool kGrouped>
-int32_t ibatch_fmt(int n_groups, int64_t n, int64_t k, const void* w, const ActPlanes& act, const int* offsets, int64_t n_rows,
+int32_t ibatch_fmt(int type, int n_groups, int64_t n, int64_t k, const void* w, const ActPlanes& act, const int* offsets, int64_t n_rows,
                    const int* out_rows, float* y, cudaStream_t stream, bool early_w) {
   DeviceInfo* di;
   if (!device_info(&di)) return kLaunchFailure;
@@ -676,14 +635,10 @@ int32_t ibatch_fmt(int n_groups, int64_t n, int64_t k, const void* w, const ActP
       if (!plan_ibatch<F>(&p, tiles, warps, (size_t)di->max_smem_optin, &smem)) return kNotSupported;
     }
   }
-  const dim3 grid((unsigned)blocks);
-  cudaError_t e;
-  if (p.rows_cap <= 8) e = launch_ibatch<F, 1, kGrouped>(p, grid, warps, smem, stream);
-  else if (p.rows_cap <= 16) e = launch_ibatch<F, 2, kGrouped>(p, grid, warps, smem, stream);
-  else if (!kGrouped && p.rows_cap <= 24) e = launch_ibatch<F, kGrouped ? 4 : 3, kGrouped>(p, grid, warps, smem, stream);
-  else if (p.rows_cap <= 32) e = launch_ibatch<F, 4, kGrouped>(p, grid, warps, smem, stream);
-  else if (!kGrouped && p.rows_cap <= 48) e = launch_ibatch<F, kGrouped ? 8 : 6, kGrouped>(p, grid, warps, smem, stream);
-  else e = launch_ibatch<F, 8, kGrouped>(p, grid, warps, smem, stream);
+  int mt = p.rows_cap / 8;
+  if (mt > 4) mt = !kGrouped && mt <= 6 ? 6 : 8;
+  if (kGrouped && mt == 3) mt = 4;
+  const cudaError_t e = ibatch_launch(type, mt, kGrouped, p, (unsigned)blocks, warps, smem, di->max_smem_optin, stream);
   return e == cudaSuccess ? kOk : kLaunchFailure;
 }
 
@@ -693,12 +648,12 @@ int32_t ibatch_impl(int type, int n_groups, int64_t n, int64_t k, const void* w,
   if (k % 256 || n > INT32_MAX - 64 || n_groups > 65535 || n_rows > (1 << 28)) return kNotSupported;
   if (!act.rec && n_rows > 1) return kNotSupported;  // planes are read for single rows only
   if (offsets) {
-    if (type == kQ4K) return ibatch_fmt<IbQ4K, true>(n_groups, n, k, w, act, offsets, n_rows, out_rows, y, stream, early_w);
-    if (type == kQ6K) return ibatch_fmt<IbQ6K, true>(n_groups, n, k, w, act, offsets, n_rows, out_rows, y, stream, early_w);
+    if (type == kQ4K) return ibatch_fmt<IbQ4K, true>(type, n_groups, n, k, w, act, offsets, n_rows, out_rows, y, stream, early_w);
+    if (type == kQ6K) return ibatch_fmt<IbQ6K, true>(type, n_groups, n, k, w, act, offsets, n_rows, out_rows, y, stream, early_w);
     return kNotSupported;
   }
 #define FQ_IB(T, F) \
-  case T: return ibatch_fmt<F, false>(n_groups, n, k, w, act, offsets, n_rows, out_rows, y, stream, early_w)
+  case T: return ibatch_fmt<F, false>(type, n_groups, n, k, w, act, offsets, n_rows, out_rows, y, stream, early_w)
   switch (type) {
     FQ_IB(kQ4K, IbQ4K);
     FQ_IB(kQ5K, IbQ5K);
@@ -1131,11 +1086,13 @@ int32_t fuelq_device_error(int32_t* host_code_out, int32_t clear) {
   int code = 0;
   if (cudaDeviceSynchronize() != cudaSuccess) return kLaunchFailure;
   if (cudaMemcpyFromSymbol(&code, g_fq_dev_error, sizeof(int)) != cudaSuccess) return kLaunchFailure;
+  int batch = 0;
+  if (ibatch_device_error(&batch, clear != 0) != cudaSuccess) return kLaunchFailure;
   if (clear && code) {
     const int zero = 0;
     if (cudaMemcpyToSymbol(g_fq_dev_error, &zero, sizeof(int)) != cudaSuccess) return kLaunchFailure;
   }
-  if (host_code_out) *host_code_out = code;
+  if (host_code_out) *host_code_out = code ? code : batch;
   return kOk;
 }
 

@@ -62,6 +62,10 @@ struct IbParams {
   int part_off;          // and of the partial sums
 };
 
+// Launches the kernel of a weight type for mt 8-row tiles (ibatch.cu)
+cudaError_t ibatch_launch(int type, int mt, bool grouped, const IbParams& p, unsigned grid, int warps, size_t smem, int max_smem, cudaStream_t stream);
+cudaError_t ibatch_device_error(int* code, bool clear);  // the error word of these kernels
+
 // ---- small pieces
 __device__ __forceinline__ void ib_cp16(uint32_t dst, const void* src, uint32_t bytes) {  // bytes past `bytes` become zero
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
