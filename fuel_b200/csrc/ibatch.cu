@@ -1,5 +1,5 @@
-// The integer batch kernels, apart from the rest of the library: compiled together with them, kernels that have nothing to do
-// with these came out slower (the 7B decode step 1915 -> 2010 us, the GEMM of 2048 rows 237 -> 255).
+// The integer batch kernels, in a translation unit of their own so that the library's two large sets of kernels compile side by
+// side.
 #include "ibatch.cuh"
 
 #include "launch.cuh"
