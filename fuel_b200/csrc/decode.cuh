@@ -89,7 +89,7 @@ struct Q4KDecode {
         dh = dp4a_ss(h1, ahi.y, dh);
         dh = dp4a_ss(h2, ahi.z, dh);
         dh = dp4a_ss(h3, ahi.w, dh);
-        const int16_t* bs = a.bsums + ((size_t)m * (k >> 8) + blk) * kSumStride + 4 * g + h;
+        const int16_t* bs = a.bsums + (size_t)m * (k >> 4) + blk * 16 + 4 * g + h;
         const int bl = bs[0], bh = bs[2];
         const float yd = a.d[(size_t)m * nblk + blk];
         acc[i] += (d * yd) * (float)(sc_lo * dl + sc_hi * dh) - (dmin * yd) * (float)(mn_lo * bl + mn_hi * bh);
@@ -302,7 +302,7 @@ struct Q2KDecode {
       if (i < mc) {
         const int m = m0 + i;
         const int8_t* q8 = a.qs + (size_t)m * k + (size_t)blk * 256 + 128 * c + 16 * h;
-        const int16_t* bs = a.bsums + ((size_t)m * (k >> 8) + blk) * kSumStride + 8 * c + h;
+        const int16_t* bs = a.bsums + (size_t)m * (k >> 4) + blk * 16 + 8 * c + h;
         int isum = 0, msum = 0;
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
@@ -352,7 +352,7 @@ struct Q3KDecode {
       if (i < mc) {
         const int m = m0 + i;
         const int8_t* q8 = a.qs + (size_t)m * k + (size_t)blk * 256 + 128 * c + 16 * h;
-        const int16_t* bs = a.bsums + ((size_t)m * (k >> 8) + blk) * kSumStride + 8 * c + h;
+        const int16_t* bs = a.bsums + (size_t)m * (k >> 4) + blk * 16 + 8 * c + h;
         int isum = 0;
 #pragma unroll
         for (int j = 0; j < 4; ++j) {

@@ -104,7 +104,7 @@ struct Q4KRegs {
       const int4 v = q8[i];
       ac.q[4 * i] = v.x, ac.q[4 * i + 1] = v.y, ac.q[4 * i + 2] = v.z, ac.q[4 * i + 3] = v.w;
     }
-    const int4 bs = *reinterpret_cast<const int4*>(a.bsums + ((size_t)m * (k >> 8) + blk) * kSumStride + 8 * h);
+    const int4 bs = *reinterpret_cast<const int4*>(a.bsums + (size_t)m * (k >> 4) + blk * 16 + 8 * h);
     set_sums(bs.x, bs.y, bs.z, bs.w, ac);
     ac.yd = a.d[(size_t)m * (k >> 8) + blk];
   }
@@ -292,7 +292,7 @@ struct Q6KRegs {
       const int4 v = q8[i];
       ac.q[4 * i] = v.x, ac.q[4 * i + 1] = v.y, ac.q[4 * i + 2] = v.z, ac.q[4 * i + 3] = v.w;
     }
-    const int4 bs = *reinterpret_cast<const int4*>(a.bsums + ((size_t)m * (k >> 8) + blk) * kSumStride + 8 * h);
+    const int4 bs = *reinterpret_cast<const int4*>(a.bsums + (size_t)m * (k >> 4) + blk * 16 + 8 * h);
     ac.bs[0] = bs.x, ac.bs[1] = bs.y, ac.bs[2] = bs.z, ac.bs[3] = bs.w;
     ac.yd = a.d[(size_t)m * (k >> 8) + blk];
   }

@@ -75,11 +75,9 @@ __host__ __device__ inline int act_type_for(int t) {
 // Q8_K / Q8_0 blocks, split into planes so every plane is 16-byte aligned:
 //   qs    int8  [m][k]
 //   d     f32   [m][k / act_block]      (for Q8_0: the f16-rounded scale widened to f32)
-//   bsums [m][k / 256] of 64 bytes: the sixteen 16-element sums as int16, then the same as f16 (at most 2048 in
-//         magnitude, so exact) for the tensor-core kernel's minimum term (Q8_K only)
+//   bsums int16 [m][k / 16]             (Q8_K only)
 //         Q8_1 instead keeps, in the same slot, f32 [m][k / 32]: the block's s = d * sum(q), f16-rounded as the
-//         reference stores it (k_quants.rs:728-757), widened to f32
-constexpr int kSumStride = 32;  // int16 units per block of the bsums plane
+//         reference stores it (k_quants.rs:728-757), widened to f32 (same byte count as the int16 plane)
 struct ActPlanes {
   const uint8_t* rec;  // not null: records at this address, and no planes
   const int8_t* qs;
@@ -88,7 +86,7 @@ struct ActPlanes {
 };
 // Two or more rows of whole 256-element stretches are kept as RECORDS instead: [k / 256][m] of kActRecord (Q8_1:
 // kActRecordMin) bytes, everything one stretch of one row brings to the tensor-core kernel (ibatch.cuh) -
-//   256 int8 | Q8_K: sixteen 16-element sums as f16, then d; Q8_0: eight d; Q8_1: eight d, eight s | padding
+//   256 int8 | Q8_K: sixteen 16-element sums as f16 (at most 2048 in magnitude, so exact), then d; Q8_0: eight d; Q8_1: eight d, eight s | padding
 // so that a stretch of all rows of a batch is ONE contiguous copy into shared memory, and so that eight consecutive records
 // start in eight different 16-byte columns of the banks (304 and 336 modulo 128 step through them all).
 constexpr int kActRecord = 304, kActRecordMin = 336, kActRecAux = 256, kActRecD = 288;
@@ -101,7 +99,7 @@ __host__ __device__ inline size_t act_packed_bytes(int weight_type, int64_t m, i
   const int at = act_type_for(weight_type);
   const int be = block_elems(at);
   size_t b = align_up((size_t)m * k, 256) + align_up((size_t)m * (k / be) * 4, 256);
-  if (at == kQ8K || at == kQ8_1) b += align_up(at == kQ8K ? (size_t)m * (k / 256) * 64 : (size_t)m * (k / 32) * 4, 256);
+  if (at == kQ8K || at == kQ8_1) b += align_up((size_t)m * (k / 16) * 2, 256);
   const size_t rec = act_records(m, k) ? (size_t)m * (k / 256) * act_record_bytes(weight_type) : 0;
   return rec > b ? rec : b;
 }

@@ -694,7 +694,7 @@ int32_t decode_chunked(int type, int64_t m_total, int64_t n, int64_t k, const vo
     a.rec = nullptr;
     a.qs = all.qs + m0 * k;
     a.d = all.d + m0 * (k / abe);
-    a.bsums = all.bsums ? all.bsums + (abe == QK_K ? m0 * (k / 256) * kSumStride : m0 * (k / 16)) : nullptr;
+    a.bsums = all.bsums ? all.bsums + m0 * (k / 16) : nullptr;
     const int32_t st = decode_impl(type, mc, n, k, w, a, y + m0 * n, stream, early_w);
     if (st != kOk) return st;
   }

@@ -132,6 +132,17 @@ __device__ __forceinline__ uint2 lds64(uint32_t a) {
   asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(a));
   return v;
 }
+__device__ __forceinline__ void ib_sums16(uint32_t dst, const int16_t* src) {  // eight sums of the plane as f16
+  const int4 v = *reinterpret_cast<const int4*>(src);
+  const int in[4] = {v.x, v.y, v.z, v.w};
+  uint32_t h[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const __half2 p = __halves2half2(__int2half_rn((int16_t)in[i]), __int2half_rn(in[i] >> 16));
+    h[i] = *reinterpret_cast<const uint32_t*>(&p);
+  }
+  asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(dst), "r"(h[0]), "r"(h[1]), "r"(h[2]), "r"(h[3]) : "memory");
+}
 __device__ __forceinline__ int ib_byte(uint32_t w, int i) { return (int)((w >> (8 * i)) & 0xffu); }
 __device__ __forceinline__ int ib_sbyte(uint32_t w, int i) { return (int)(int8_t)((w >> (8 * i)) & 0xffu); }
 __device__ __forceinline__ uint32_t ib_h2(int a, int b) {  // two small integers as packed f16
@@ -190,6 +201,7 @@ struct IbQ45K {
   static constexpr int kBytes256 = kFive ? 176 : 144, kPitch = kBytes256;  // 144 and 176 both spread eight rows over the banks
   static constexpr bool kAligned = true;
   static constexpr IbAct kAct = kIbQ8K;
+  static constexpr bool kSums = true;  // reads the 16-element sums
   template <int NT, bool kSingly, int MT>
   __device__ __forceinline__ static void block(const IbCtx& cx, float (&facc)[MT][4]) {
     const uint4 h0 = lds128(cx.r0), h1 = lds128(cx.r1);
@@ -282,6 +294,7 @@ struct IbQ6K {
   static constexpr int kBytes256 = 210, kPitch = 240;  // fetched as 14 16-byte pieces (skew 0..14)
   static constexpr bool kAligned = false;
   static constexpr IbAct kAct = kIbQ8K;
+  static constexpr bool kSums = false;
   template <int NT, bool kSingly, int MT>
   __device__ __forceinline__ static void block(const IbCtx& cx, float (&facc)[MT][4]) {
     int S[NT][4];
@@ -322,6 +335,7 @@ struct IbQ3K {
   static constexpr int kBytes256 = 110, kPitch = 144;  // fetched as eight pieces
   static constexpr bool kAligned = false;
   static constexpr IbAct kAct = kIbQ8K;
+  static constexpr bool kSums = false;
   __device__ __forceinline__ static void scales(uint32_t row, uint32_t (&sc)[4]) {  // k_quants.rs:1095-1103, minus 32 per byte
     const uint32_t a = lds_u32_2b_addr(row + 96u), b = lds_u32_2b_addr(row + 100u), c = lds_u32_2b_addr(row + 104u);
     sc[0] = (a & 0x0f0f0f0fu) | ((c & 0x03030303u) << 4);
@@ -374,6 +388,7 @@ struct IbQ2K {
   static constexpr int kBytes256 = 84, kPitch = 112;  // fetched as six or seven pieces (skew 0, 4, 8, 12)
   static constexpr bool kAligned = false;
   static constexpr IbAct kAct = kIbQ8K;
+  static constexpr bool kSums = true;
   template <int NT, bool kSingly, int MT>
   __device__ __forceinline__ static void block(const IbCtx& cx, float (&facc)[MT][4]) {
     uint32_t am[4], sw[2][4];
@@ -724,7 +739,7 @@ __global__ void __launch_bounds__(32 * (MT > 4 ? kIbMaxWarps / 2 : kIbMaxWarps),
         const uint32_t dst = smem + base + (uint32_t)(s * slot_bytes);
         ib_cp16(dst + 16u * piece, p.act.qs + b * 256 + 16 * piece, 16u);
         if constexpr (F::kAct == kIbQ8K) {
-          if (piece < 2) ib_cp16(dst + kActRecAux + 16u * piece, p.act.bsums + b * kSumStride + 16 + 8 * piece, 16u);  // the f16 form
+          if (F::kSums && piece < 2) ib_sums16(dst + kActRecAux + 16u * piece, p.act.bsums + b * 16 + 8 * piece);
           else if (piece == 2) ib_cp4(dst + kActRecD, p.act.d + b, 4u);
         } else {
           if (piece < 2) ib_cp16(dst + kActRecAux + 16u * piece, p.act.d + b * 8 + 4 * piece, 16u);

@@ -330,7 +330,7 @@ __global__ void __launch_bounds__(kDecodeThreads, 2) moe_decode_kernel(const Moe
   // ---------------- consumers
   const ActPlanes sp = act_planes(smem_raw + p.act_smem_off, kQ4K, p.act_rows, p.k);
   const int t = threadIdx.x, nt = 32 * kDecodeConsumerWarps;
-  const int dpr = p.k >> 8, bpr = dpr * kSumStride;  // block scales / int16 units of the sums plane per row
+  const int dpr = p.k >> 8, bpr = p.k >> 4;  // block scales / 16-sums per row
   int g = 0;
   for (int pass = 0; pass < n_pass; ++pass) {
     const int a0 = m_begin + pass * p.act_rows;
@@ -342,7 +342,7 @@ __global__ void __launch_bounds__(kDecodeThreads, 2) moe_decode_kernel(const Moe
         const uint8_t* rec = p.act.rec + ((size_t)b * p.n_rows + a0 + r) * kActRecord;
         for (int j = 0; j < 16; ++j) reinterpret_cast<uint4*>(const_cast<int8_t*>(sp.qs) + (size_t)r * p.k + b * 256)[j] = reinterpret_cast<const uint4*>(rec)[j];
         const_cast<float*>(sp.d)[(size_t)r * dpr + b] = *reinterpret_cast<const float*>(rec + kActRecD);
-        int16_t* bs = const_cast<int16_t*>(sp.bsums) + ((size_t)r * dpr + b) * kSumStride;
+        int16_t* bs = const_cast<int16_t*>(sp.bsums) + ((size_t)r * dpr + b) * 16;
         for (int j = 0; j < 16; ++j) bs[j] = (int16_t)__half2int_rn(reinterpret_cast<const __half*>(rec + kActRecAux)[j]);
       }
     } else {

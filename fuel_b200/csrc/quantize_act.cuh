@@ -81,13 +81,6 @@ __device__ __forceinline__ Q8KLaneBlock q8k_block_quantize(const float (&e)[8], 
   return b;
 }
 
-// sums of 16-element groups g and 8 + g, in both forms of the plane
-__device__ __forceinline__ void store_sums(int16_t* out, int g, int s0, int s1) {
-  out[g] = (int16_t)s0, out[8 + g] = (int16_t)s1;
-  __half* h = reinterpret_cast<__half*>(out + 16);
-  h[g] = __int2half_rn(s0), h[8 + g] = __int2half_rn(s1);
-}
-
 __device__ __forceinline__ void q8k_block_store(const Q8KLaneBlock& b, int lane, int64_t blk, int8_t* out_qs,
                                                 float* out_d, int16_t* out_bsums) {
   uint32_t* qs = reinterpret_cast<uint32_t*>(out_qs + blk * QK_K);
@@ -95,7 +88,8 @@ __device__ __forceinline__ void q8k_block_store(const Q8KLaneBlock& b, int lane,
   qs[32 + lane] = b.p1;
   if (lane == 0) out_d[blk] = b.d;
   if ((lane & 3) == 0) {
-    store_sums(out_bsums + blk * kSumStride, lane >> 2, b.s0, b.s1);
+    out_bsums[blk * 16 + (lane >> 2)] = (int16_t)b.s0;
+    out_bsums[blk * 16 + 8 + (lane >> 2)] = (int16_t)b.s1;
   }
 }
 

@@ -144,3 +144,13 @@ def test_argument_validation_of_moe_and_peer_entries_needs_no_gpu():
     peers.world, peers.rank = 2, 2
     assert L.fuelq_argmax_last_peer(16, 8, 16, ctypes.byref(peers), 0, 16, None) == INV                              # rank >= world
     assert L.fuelq_peer_vec_bytes(10) == 80
+
+
+def test_single_rows_hold_their_sums_once():
+    """One row's Q8_K blocks: values, scales and 16-element sums (int16), each from a 256-byte boundary; a second form of the
+    sums would make every kernel of a decode step that quantizes write it."""
+    from fuel_b200 import _lib as L
+    for k in (256, 4096, 11008):
+        up = lambda b: -(-b // 256) * 256
+        for fmt in (10, 11, 12, 13, 14):
+            assert L.lib.fuelq_act_packed_bytes(fmt, 1, k) == up(k) + up(k // 256 * 4) + up(k // 16 * 2)

@@ -41,6 +41,7 @@ def test_batch_edges_match_the_oracle(oracle, name):
     ([1] * 70 + [0] * 5 + [40] + [2] * 52, 37, 512),          # many: blocks that span several, one group in several passes
     ([17, 0, 33, 24, 8, 130, 1, 16] * 5, 165, 2304),          # up to 64 rows a pass, and more
     ([26, 31, 12, 0, 25, 18, 32, 20] * 16, 85, 2048),         # some twenty rows each: sixteen warps a block
+    ([0, 0, 1, 0], 37, 1280),                                 # a single row: planes, the sums converted as they are staged
 ])
 def test_groups_match_the_oracle(oracle, name, counts, n, k):
     if not torch.cuda.is_available():
