@@ -232,9 +232,9 @@ static __global__ void __launch_bounds__(32) prefetch_l2_kernel(const uint8_t* _
 
 
 // n f32 words from device memory to a device-mapped host buffer (or any other place), 16 bytes per thread where
-// both addresses allow it: the write-back of a small result without a copy-engine hand-off.
-static __global__ void __launch_bounds__(256) copy_out_f32_kernel(const float* __restrict__ src, float* __restrict__ dst, long long n,
-                                                           int vec) {
+// both addresses allow it: the write-back of a small result without a copy-engine hand-off. src is what the kernel before
+// this one writes: not __restrict__, which would let its loads move above the wait.
+static __global__ void __launch_bounds__(256) copy_out_f32_kernel(const float* src, float* dst, long long n, int vec) {
   pdl_launch_dependents();
   pdl_wait();
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x, nt = (long long)gridDim.x * blockDim.x;
