@@ -8,7 +8,6 @@
 #include <cstddef>
 #include <cstring>
 #include <map>
-#include <unordered_map>
 
 #include "../../include/fuelq.h"
 #include "../../include/fuelq_seam.h"
@@ -23,70 +22,6 @@ void cuda_check(cudaError_t e, const char* op) {
   if (e != cudaSuccess) throw Error(std::string(op) + ": " + cudaGetErrorString(e), FUELQ_LAUNCH_FAILURE);
 }
 cudaStream_t cs(const Device& d) { return static_cast<cudaStream_t>(d.stream()); }
-
-// Freed device blocks kept for the next allocation of about their size. cudaMalloc and cudaFree map and unmap memory: 0.5 to
-// 60 ms each was measured for a 9 MB matrix on a shared host, against microseconds for quantizing one, so a program that
-// converts or swaps weights spent its time there. At most kMostBytes per device are kept; what does not fit goes back to
-// the driver at once, and everything kept does when an allocation fails.
-class BlockCache {
- public:
-  static constexpr size_t kMostBytes = (size_t)512 << 20, kGranule = (size_t)2 << 20;
-  static BlockCache& instance() {
-    static BlockCache* c = new BlockCache;  // never destroyed: buffers may be released during process exit
-    return *c;
-  }
-  // small blocks keep their size: the driver packs them into one granule
-  static size_t rounded(size_t bytes) { return bytes < kGranule / 2 ? std::max<size_t>(bytes, 16) : (bytes + kGranule - 1) / kGranule * kGranule; }
-  cudaError_t take(int ordinal, size_t bytes, void** out) {  // the device is current
-    {
-      std::lock_guard<std::mutex> lock(mu_);
-      auto& free = free_[ordinal];
-      auto it = free.lower_bound(bytes);
-      if (it != free.end() && it->first <= bytes + bytes / 8) {
-        *out = it->second;
-        kept_[ordinal] -= it->first;
-        sizes_[*out] = it->first;
-        free.erase(it);
-        return cudaSuccess;
-      }
-    }
-    cudaError_t e = cudaMalloc(out, bytes);
-    if (e == cudaErrorMemoryAllocation) {
-      cudaGetLastError();
-      flush(ordinal);
-      e = cudaMalloc(out, bytes);
-    }
-    if (e == cudaSuccess) {
-      std::lock_guard<std::mutex> lock(mu_);
-      sizes_[*out] = bytes;
-    }
-    return e;
-  }
-  void give(int ordinal, void* p) {  // the device is current; like cudaFree, waits for work that may still use the block
-    const bool idle = cudaDeviceSynchronize() == cudaSuccess;
-    std::lock_guard<std::mutex> lock(mu_);
-    const size_t bytes = sizes_[p];
-    sizes_.erase(p);
-    if (idle && kept_[ordinal] + bytes <= kMostBytes) {
-      free_[ordinal].emplace(bytes, p);
-      kept_[ordinal] += bytes;
-    } else {
-      cudaFree(p);
-    }
-  }
-
- private:
-  void flush(int ordinal) {
-    std::lock_guard<std::mutex> lock(mu_);
-    for (auto& b : free_[ordinal]) cudaFree(b.second);
-    free_[ordinal].clear();
-    kept_[ordinal] = 0;
-  }
-  std::mutex mu_;
-  std::map<int, std::multimap<size_t, void*>> free_;
-  std::map<int, size_t> kept_;
-  std::unordered_map<void*, size_t> sizes_;
-};
 }  // namespace
 
 size_t type_size(GgmlDType t) {
@@ -124,13 +59,13 @@ void Device::synchronize() const {
 
 DeviceBuffer::DeviceBuffer(const Device& dev, size_t bytes, bool zero) : bytes_(bytes), ordinal_(dev.ordinal()) {
   dev.make_current();
-  cuda_check(BlockCache::instance().take(ordinal_, BlockCache::rounded(bytes), &ptr_), "cudaMalloc");
+  cuda_check(cudaMalloc(&ptr_, bytes ? bytes : 16), "cudaMalloc");
   if (zero && bytes) cuda_check(cudaMemsetAsync(ptr_, 0, bytes, static_cast<cudaStream_t>(dev.stream())), "cudaMemset");
 }
 DeviceBuffer::~DeviceBuffer() {
   if (ptr_) {
     cudaSetDevice(ordinal_);
-    BlockCache::instance().give(ordinal_, ptr_);
+    cudaFree(ptr_);
   }
 }
 DeviceBuffer::DeviceBuffer(DeviceBuffer&& o) noexcept : ptr_(o.ptr_), bytes_(o.bytes_), ordinal_(o.ordinal_) {
@@ -141,7 +76,7 @@ DeviceBuffer& DeviceBuffer::operator=(DeviceBuffer&& o) noexcept {
   if (this != &o) {
     if (ptr_) {
       cudaSetDevice(ordinal_);
-      BlockCache::instance().give(ordinal_, ptr_);
+      cudaFree(ptr_);
     }
     ptr_ = o.ptr_, bytes_ = o.bytes_, ordinal_ = o.ordinal_;
     o.ptr_ = nullptr, o.bytes_ = 0;
