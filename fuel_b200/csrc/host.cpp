@@ -149,15 +149,38 @@ std::vector<uint8_t> QStorage::data() const {
   return out;
 }
 
+// The legacy default stream needs no query: there is one of it, and it can't be captured.
+static bool is_legacy(const Device& dev) { return !dev.stream() || cs(dev) == cudaStreamLegacy; }
+static uint64_t stream_id(const Device& dev) {  // the device is current, unless the stream is the legacy one
+  unsigned long long id = ~0ull;
+  if (!is_legacy(dev)) cuda_check(cudaStreamGetId(cs(dev), &id), "cudaStreamGetId");
+  return id;
+}
+
 std::shared_ptr<SharedWorkspace> SharedWorkspace::of(const Device& dev) {
   static std::mutex mu;
-  static std::map<std::pair<int, void*>, std::weak_ptr<SharedWorkspace>> all;
+  static std::map<std::pair<int, uint64_t>, std::weak_ptr<SharedWorkspace>> all;
+  if (!is_legacy(dev)) dev.make_current();
+  const uint64_t id = fuelq::stream_id(dev);
   std::lock_guard<std::mutex> lock(mu);
   for (auto it = all.begin(); it != all.end();) it = it->second.expired() ? all.erase(it) : std::next(it);
-  std::weak_ptr<SharedWorkspace>& slot = all[{dev.ordinal(), dev.stream()}];
+  std::weak_ptr<SharedWorkspace>& slot = all[{dev.ordinal(), id}];
   std::shared_ptr<SharedWorkspace> ws = slot.lock();
-  if (!ws) slot = ws = std::make_shared<SharedWorkspace>();
+  if (!ws) slot = ws = std::make_shared<SharedWorkspace>(), ws->stream_id = id;
   return ws;
+}
+void SharedWorkspace::enter(const Device& dev) {
+  cudaEvent_t e = static_cast<cudaEvent_t>(last_use);
+  if (!e) {
+    cuda_check(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "cudaEventCreate");
+    last_use = e;
+  } else {
+    cuda_check(cudaStreamWaitEvent(cs(dev), e, 0), "cudaStreamWaitEvent");
+  }
+}
+void SharedWorkspace::leave(const Device& dev) { cuda_check(cudaEventRecord(static_cast<cudaEvent_t>(last_use), cs(dev)), "cudaEventRecord"); }
+SharedWorkspace::~SharedWorkspace() {
+  if (last_use) cudaEventDestroy(static_cast<cudaEvent_t>(last_use));
 }
 void* SharedWorkspace::ensure(const Device& dev, size_t need, size_t least) {
   if (bytes() < need || buffers.empty()) {
@@ -180,21 +203,22 @@ void QStorage::fwd_into(const Shape& self_shape, const float* x, const Shape& in
   fwd_rows(n, k, x, elem_count(in_shape) / (k ? k : 1), y);
 }
 
-// The legacy default stream can't be captured, so the usual caller is spared the query.
 static bool capturing(const Device& dev) {
   cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
-  return dev.stream() && cs(dev) != cudaStreamLegacy && cudaStreamIsCapturing(cs(dev), &status) == cudaSuccess &&
-         status == cudaStreamCaptureStatusActive;
+  return !is_legacy(dev) && cudaStreamIsCapturing(cs(dev), &status) == cudaSuccess && status == cudaStreamCaptureStatusActive;
 }
 
 void QStorage::fwd_rows(int64_t n, int64_t k, const float* x, int64_t m, float* y) const {
   dev_.make_current();
   const size_t need = fuelq_qmatmul_workspace_bytes((int32_t)dtype_, m, n, k);
-  const bool recorded = capturing(dev_);
-  SharedWorkspace& ws = recorded ? *captured_ : *workspace_;
+  const bool recorded = capturing(dev_), elsewhere = !recorded && stream_id(dev_) != workspace_->stream_id;
+  SharedWorkspace& ws = recorded ? *captured_ : elsewhere ? *elsewhere_ : *workspace_;
   std::lock_guard<std::mutex> lock(ws.mutex);
-  void* scratch = ws.ensure(dev_, need, recorded ? 16 : (size_t)1 << 20);
-  check(fuelq_qmatmul((int32_t)dtype_, m, n, k, buf_.ptr(), x, y, scratch, ws.bytes(), dev_.stream()), "fuelq_qmatmul");
+  void* scratch = ws.ensure(dev_, need, recorded || elsewhere ? 16 : (size_t)1 << 20);
+  if (elsewhere) ws.enter(dev_);
+  const int32_t status = fuelq_qmatmul((int32_t)dtype_, m, n, k, buf_.ptr(), x, y, scratch, ws.bytes(), dev_.stream());
+  if (elsewhere) ws.leave(dev_);
+  check(status, "fuelq_qmatmul");
 }
 
 std::pair<DeviceBuffer, Shape> QStorage::fwd(const Shape& self_shape, const float* x, const Shape& in_shape) const {

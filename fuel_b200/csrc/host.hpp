@@ -78,18 +78,29 @@ class DeviceBuffer {
   int ordinal_ = 0;
 };
 
-// Device scratch for fwd, shared by every storage on one (device, stream), calls under stream capture aside: the calls of a stream run in order, so one buffer
-// serves all of a model's linears (one each would cost a model of two hundred of them gigabytes, and an allocation with a
-// device synchronization on each one's first call). Growing keeps the smaller buffers, since kernels in flight or captured
-// graphs may hold their addresses; growth is at least twofold, so the total stays below twice the largest need, and all of
-// it is released with the last storage that uses it. A caller holds `mutex` while it enqueues the kernels of one product, so
-// that two threads on one stream do not interleave theirs.
+// Device scratch for fwd, shared by every storage made on one stream: the calls of a stream run in order, so one buffer serves
+// all of a model's linears (one each would cost a model of two hundred of them gigabytes, and an allocation with a device
+// synchronization on each one's first call). Streams are told apart by their id, which is never given out twice: a handle
+// is, after its stream is destroyed, and cudaStreamPerThread is one handle for a stream of every thread. Growing keeps the
+// smaller buffers, since kernels in flight or captured graphs may hold their addresses; growth is at least twofold, so the
+// total stays below four times the largest need, and all of it is released with the last storage that uses it. A caller
+// holds `mutex` while it enqueues the kernels of one product, so that two threads on one stream do not interleave theirs.
 struct SharedWorkspace {
   std::mutex mutex;
   std::vector<DeviceBuffer> buffers;  // the last one is the largest
+  uint64_t stream_id = 0;             // the one it is shared on
+  void* last_use = nullptr;           // event, where calls come from several streams
   static std::shared_ptr<SharedWorkspace> of(const Device& dev);
-  void* ensure(const Device& dev, size_t bytes, size_t least);  // with `mutex` held; at least `least` when it allocates
+  // With `mutex` held; at least `least` bytes when it allocates
+  void* ensure(const Device& dev, size_t bytes, size_t least);
   size_t bytes() const { return buffers.empty() ? 0 : buffers.back().bytes(); }
+  // With `mutex` held, around the kernels of a call: they run after those of the call before it, whatever its stream
+  void enter(const Device& dev);
+  void leave(const Device& dev);
+  SharedWorkspace() = default;
+  SharedWorkspace(const SharedWorkspace&) = delete;
+  SharedWorkspace& operator=(const SharedWorkspace&) = delete;
+  ~SharedWorkspace();
 };
 
 class QStorage {
@@ -138,6 +149,9 @@ class QStorage {
   // Calls recorded into a graph get scratch of this storage alone: the graph may be replayed on another stream, beside the
   // calls that share workspace_.
   std::unique_ptr<SharedWorkspace> captured_ = std::make_unique<SharedWorkspace>();
+  // So do calls whose handle names another stream by now than the one workspace_ belongs to: cudaStreamPerThread in another
+  // thread, or a handle that was given out again. They wait for one another.
+  std::unique_ptr<SharedWorkspace> elsewhere_ = std::make_unique<SharedWorkspace>();
 };
 
 class QTensor {
