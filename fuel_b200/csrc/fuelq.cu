@@ -701,6 +701,20 @@ int32_t decode_chunked(int type, int64_t m_total, int64_t n, int64_t k, const vo
   return kOk;
 }
 
+// Packed rows under FUELQ_OPT_DECODE_KERNEL: its kernels read planes, a caller's buffer of several rows holds records. The
+// planes are stream-ordered memory for the length of the call.
+int32_t decode_forced(int type, int64_t m_total, int64_t n, int64_t k, const void* w, const void* packed_act, float* y, cudaStream_t stream) {
+  void* planes = nullptr;
+  if (cudaMallocAsync(&planes, act_packed_bytes(type, m_total, k), stream) != cudaSuccess) return kLaunchFailure;
+  const ActPlanes a = act_planes(planes, type, m_total, k);
+  const int64_t n_rec = m_total * (k / 256);
+  const cudaError_t e = launch(records_to_planes_kernel, dim3((unsigned)((n_rec + 7) / 8)), dim3(256), 0, stream, (const uint8_t*)packed_act,
+                               (int)m_total, n_rec, act_record_bytes(type), act_type_for(type), (int8_t*)a.qs, (float*)a.d, (int16_t*)a.bsums);
+  const int32_t st = e == cudaSuccess ? decode_chunked(type, m_total, n, k, w, planes, y, stream, false, true) : (int32_t)kLaunchFailure;
+  if (cudaFreeAsync(planes, stream) != cudaSuccess) return kLaunchFailure;
+  return st;
+}
+
 // ---- block -> float dequantization (dequantize.cuh)
 // out_type: kF32, kF16, kBF16, or the tensor-core path's operands: kF16Sat (f16 with finite overflow saturated) and
 // kTf32 (f32 rounded to tf32)
@@ -1148,6 +1162,8 @@ int32_t fuelq_qmatmul_packed(int32_t ggml_type, int64_t m_total, int64_t n, int6
     const int32_t sp = prefetch_impl(w, n * (k / block_elems(ggml_type)) * block_bytes(ggml_type), (cudaStream_t)stream);
     if (sp != kOk) return sp;
   }
+  if (integer_kernel_forced() && act_records(m_total, k))
+    return decode_forced(ggml_type, m_total, n, k, w, packed_act, y, (cudaStream_t)stream);
   return decode_chunked(ggml_type, m_total, n, k, w, const_cast<void*>(packed_act), y, (cudaStream_t)stream, false);
 }
 

@@ -282,4 +282,25 @@ __global__ void __launch_bounds__(256) quantize_q8_0_kernel(const float* x, int6
   }
 }
 
+// Records (fq_common.cuh) to the planes of the same rows, one warp per record: for the kernels that an option forces on a
+// caller's packed rows. The f16 sums are whole numbers.
+static __global__ void __launch_bounds__(256) records_to_planes_kernel(const uint8_t* rec, int rows, int64_t n_rec, int rec_bytes, int act_type,
+                                                                int8_t* qs, float* d, int16_t* bsums) {
+  pdl_wait();
+  const int lane = threadIdx.x & 31;
+  const int64_t i = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);  // stretch * rows + row
+  if (i >= n_rec) return;
+  const int64_t b = i / rows, row = i - b * rows, blk = row * (n_rec / rows) + b;
+  const uint8_t* r = rec + i * rec_bytes;
+  reinterpret_cast<uint2*>(qs + blk * 256)[lane] = reinterpret_cast<const uint2*>(r)[lane];
+  if (act_type == kQ8K) {
+    if (lane < 16) bsums[blk * 16 + lane] = (int16_t)__half2int_rn(reinterpret_cast<const __half*>(r + kActRecAux)[lane]);
+    else if (lane == 16) d[blk] = *reinterpret_cast<const float*>(r + kActRecD);
+  } else {
+    const float* aux = reinterpret_cast<const float*>(r + kActRecAux);
+    if (lane < 8) d[blk * 8 + lane] = aux[lane];
+    else if (lane < 16 && act_type == kQ8_1) reinterpret_cast<float*>(bsums)[blk * 8 + lane - 8] = aux[lane];
+  }
+}
+
 }  // namespace fq

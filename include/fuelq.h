@@ -66,7 +66,9 @@ int32_t fuelq_block_bytes(int32_t ggml_type);
                                     Any positive value is taken as given */
 #define FUELQ_OPT_DECODE_GRID 3  /* CTAs for the decode kernel; 0 = two per SM (default) */
 #define FUELQ_OPT_DECODE_KERNEL 4 /* 0 = pick per problem (default); 1 = generic decode kernel (activations read
-                                    through L1, any M <= 16); 2 = register-resident kernel only (M <= 2) */
+                                    through L1, any M <= 16); 2 = register-resident kernel only (M <= 2). 1 and 2 read
+                                    another activation layout than the default's: fuelq_qmatmul_packed then takes
+                                    stream-ordered device memory for the length of the call */
 #define FUELQ_OPT_L2_PREFETCH 5   /* 1: every mat-vec call first enqueues a small kernel that streams its weight
                                     matrix from HBM into L2; with FUELQ_OPT_PDL it runs beside the preceding
                                     kernels, so the transfer overlaps their work (default 0) */

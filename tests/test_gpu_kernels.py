@@ -219,6 +219,26 @@ def test_packed_activations_are_shared(ops, oracle):
     assert torch.equal(y, ops.qmatmul(T.Q6K, wb, n, x))
 
 
+@pytest.mark.parametrize("option,name", [(1, "Q4K"), (1, "Q3K"), (1, "Q4_0"), (1, "Q5_1"), (2, "Q4K"), (2, "Q5K"), (2, "Q8_0")])
+def test_packed_activations_take_the_forced_kernel(ops, option, name):
+    """FUELQ_OPT_DECODE_KERNEL picks the same kernel for packed rows as for f32 rows: the same bits."""
+    from fuel_b200 import GgmlDType as T, _lib
+    t, n, k = getattr(T, name), 200, 2816
+    wb = ops.quantize_weights(t, _dev(_weights(n, k)))
+    for m in (1, 2, 3, 16):
+        x = _dev(_acts(m, k))
+        packed = ops.quantize_act_packed(t, x)
+        y = torch.empty(m, n, dtype=torch.float32, device="cuda")
+        try:
+            _lib.check(_lib.lib.fuelq_set_option(_lib.OPT_DECODE_KERNEL, option), "set_option")
+            want = ops.qmatmul(t, wb, n, x)
+            ops.qmatmul_packed(t, wb, n, k, m, packed, y)
+        finally:
+            _lib.lib.fuelq_set_option(_lib.OPT_DECODE_KERNEL, 0)
+        assert torch.equal(y, want), m
+    assert ops.device_error() == 0
+
+
 def test_pdl_launch_gives_same_bits(ops, oracle):
     from fuel_b200 import GgmlDType as T, _lib
     n, k = 1024, 4096
