@@ -614,16 +614,18 @@ int32_t ibatch_fmt(int type, int n_groups, int64_t n, int64_t k, const void* w, 
     if (blocks > n_tiles) blocks = n_tiles;
     if (!plan_ibatch<F>(&p, (int)((n_tiles + blocks - 1) / blocks), warps, (size_t)di->max_smem_optin, &smem)) return kNotSupported;
   } else {
-    // Routed rows: enough rows per pass for most groups (their mean and twice its root). Two thread blocks of eight warps per
+    // Routed rows: enough rows per pass for most groups (their mean and twice its root), but at most 32: the forms for more
+    // take the registers of a whole SM for eight warps (8 experts of 768 x 2048, 256 tokens, top 8, Q4_K: one block of it an
+    // SM 205 us a MoE block, two passes of 32 rows 197; Q6_K 236 and 285, but 140 and 129 at 16 experts, top 4). Two thread blocks of eight warps per
     // SM, so that one computes while the other stages, where the rows of a whole pass fit half the shared memory; else one
     // of sixteen, which fits twice as many: staged in chunks, every round of tiles would fetch them again. The kernel
     // deals the tiles of the groups that have rows out evenly; a grid per group left the SMs to wait for the largest groups,
     // and for blocks of groups without rows.
     const double mean = (double)n_rows / n_groups;
     int cap = ((int)(mean + 2.0 * sqrt(mean)) + 8) & ~7;
-    p.rows_cap = cap < 8 ? 8 : cap > kIbMaxRows ? kIbMaxRows : cap;
+    p.rows_cap = cap < 8 ? 8 : cap > kIbGroupRows ? kIbGroupRows : cap;
     const size_t half = ((size_t)di->max_smem_optin + 1024) / 2 - 1024, share = (size_t)3 * 16 * F::kPitch * (kIbMaxWarps / 2);
-    const bool two = p.rows_cap > 32 || (size_t)p.rows_cap * p.nblk * ib_rec(F::kAct) + share + 4096 <= half;
+    const bool two = (size_t)p.rows_cap * p.nblk * ib_rec(F::kAct) + share + 4096 <= half;
     if (two) warps = kIbMaxWarps / 2;
     const int64_t all = n_tiles * (n_rows < n_groups ? n_rows : n_groups);
     if (g_opt.decode_grid == 0 && two) blocks = 2 * di->sm_count;
@@ -636,7 +638,7 @@ int32_t ibatch_fmt(int type, int n_groups, int64_t n, int64_t k, const void* w, 
     }
   }
   int mt = p.rows_cap / 8;
-  if (mt > 4) mt = !kGrouped && mt <= 6 ? 6 : 8;
+  if (mt > 4) mt = mt <= 6 ? 6 : 8;
   if (kGrouped && mt == 3) mt = 4;
   const cudaError_t e = ibatch_launch(type, mt, kGrouped, p, (unsigned)blocks, warps, smem, di->max_smem_optin, stream);
   return e == cudaSuccess ? kOk : kLaunchFailure;

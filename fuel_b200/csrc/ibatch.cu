@@ -8,6 +8,8 @@ namespace fq {
 namespace {
 template <class F, int MT, bool kGrouped>
 cudaError_t launch_kernel(const IbParams& p, unsigned grid, int warps, size_t smem, int max_smem, cudaStream_t stream) {
+  // the plan deals the groups out over two thread blocks of eight warps an SM: registers for sixteen
+  static_assert(!kGrouped || MT <= kIbGroupRows / 8, "wider forms have registers for eight warps only");
   static bool attr_set[64] = {};
   auto kern = ibatch_kernel<F, MT, kGrouped>;
   int dev = 0;
@@ -39,7 +41,6 @@ cudaError_t launch_groups(int mt, const IbParams& p, unsigned grid, int warps, s
     case 1: return launch_kernel<F, 1, true>(p, grid, warps, smem, max_smem, stream);
     case 2: return launch_kernel<F, 2, true>(p, grid, warps, smem, max_smem, stream);
     case 4: return launch_kernel<F, 4, true>(p, grid, warps, smem, max_smem, stream);
-    case 8: return launch_kernel<F, 8, true>(p, grid, warps, smem, max_smem, stream);
     default: return cudaErrorInvalidValue;
   }
 }

@@ -36,6 +36,7 @@ namespace fq {
 constexpr int kIbMaxWarps = 16;
 constexpr int kIbHeader = 128;    // barriers, at the start of shared memory
 constexpr int kIbMaxRows = 64;    // activation rows per pass
+constexpr int kIbGroupRows = 32;  // and of the grouped form
 
 enum IbAct { kIbQ8K, kIbQ8_0, kIbQ8_1 };
 __host__ __device__ constexpr int ib_rec(IbAct a) { return a == kIbQ8_1 ? kActRecordMin : kActRecord; }  // bytes per row of a slot
@@ -166,13 +167,12 @@ struct IbCtx {
 // The activation tiles of a step, in parts that run together: with a branch around each tile, none of one tile's loads and
 // products can be issued under the latency of another's (Q4_K 11008 x 4096, 48 rows: 45 us, with parts 36); with all of eight,
 // or three of the sixteen-group formats at the sixteen-warp form's 128 registers, the registers spill (64 rows: 51 and 77 us).
-// kSingly: a branch around each tile all the same (the grouped form for up to 64 rows, where any number of tiles occurs).
-__host__ __device__ constexpr int ib_part(int nt, bool singly, int small, int large) {
-  return singly ? 1 : nt <= 2 ? nt : nt <= 4 ? (small < nt ? small : nt) : nt <= 6 ? nt : large;
+__host__ __device__ constexpr int ib_part(int nt, int small, int large) {
+  return nt <= 2 ? nt : nt <= 4 ? (small < nt ? small : nt) : nt <= 6 ? nt : large;
 }
 #define FQ_IB_TILES(SMALL, LARGE)                                                                                  \
-  _Pragma("unroll") for (int mq = 0; mq < NT; mq += ib_part(NT, kSingly, SMALL, LARGE)) if (mq == 0 || mq < cx.nt) \
-      _Pragma("unroll") for (int mt = mq; mt < NT && mt < mq + ib_part(NT, kSingly, SMALL, LARGE); ++mt)
+  _Pragma("unroll") for (int mq = 0; mq < NT; mq += ib_part(NT, SMALL, LARGE)) if (mq == 0 || mq < cx.nt) \
+      _Pragma("unroll") for (int mt = mq; mt < NT && mt < mq + ib_part(NT, SMALL, LARGE); ++mt)
 
 // Quant fragments of activation tile mt for 64 elements from element 64 * g: b[0..1] the first 32, b[2..3] the second
 template <int kRec = kActRecord>
@@ -202,7 +202,7 @@ struct IbQ45K {
   static constexpr bool kAligned = true;
   static constexpr IbAct kAct = kIbQ8K;
   static constexpr bool kSums = true;  // reads the 16-element sums
-  template <int NT, bool kSingly, int MT>
+  template <int NT, int MT>
   __device__ __forceinline__ static void block(const IbCtx& cx, float (&facc)[MT][4]) {
     const uint4 h0 = lds128(cx.r0), h1 = lds128(cx.r1);
     // eight 6-bit scales / mins per row as bytes of two words (get_scale_min_k4, fuel-quantized/src/utils.rs:50-60)
@@ -260,7 +260,7 @@ using IbQ5K = IbQ45K<true>;
 // ------------------------------------------------------------------------------------------------ Q6_K, Q3_K
 // Sixteen groups of 16 elements, each with a signed scale (bytes of sc0 / sc1 for rows gid / gid + 8): step g takes groups
 // 4g .. 4g + 3, A[i] = the left-justified values of group 4g + i
-template <int NT, bool kSingly>
+template <int NT>
 __device__ __forceinline__ void ib_groups16_step(const IbCtx& cx, int g, const uint32_t (&A)[4][2], uint32_t sc0, uint32_t sc1, int (&S)[NT][4]) {
   int s0[4], s1[4];
 #pragma unroll
@@ -278,7 +278,7 @@ __device__ __forceinline__ void ib_groups16_step(const IbCtx& cx, int g, const u
     }
   }
 }
-template <int NT, bool kSingly, int MT>
+template <int NT, int MT>
 __device__ __forceinline__ void ib_groups16_finish(const IbCtx& cx, const int (&S)[NT][4], float d0, float d1, float (&facc)[MT][4]) {
   FQ_IB_TILES(2, 4) {
     const uint32_t da = cx.act + (uint32_t)(8 * mt + 2 * cx.tig) * kActRecord + kActRecD;
@@ -295,7 +295,7 @@ struct IbQ6K {
   static constexpr bool kAligned = false;
   static constexpr IbAct kAct = kIbQ8K;
   static constexpr bool kSums = false;
-  template <int NT, bool kSingly, int MT>
+  template <int NT, int MT>
   __device__ __forceinline__ static void block(const IbCtx& cx, float (&facc)[MT][4]) {
     int S[NT][4];
     // 4 * (q - 32) of quadrant q of half h: elements 128 h + 32 q + l (k_quants.rs:2170-2185), l = 16 s + 4 tig .. + 3
@@ -323,11 +323,11 @@ struct IbQ6K {
             A[2 + s][r] = ((b & 0x3c3c3c3cu) ^ 0x80808080u) ^ (hb & 0xc0c0c0c0u);
           }
         const int g = 2 * h + u;
-        ib_groups16_step<NT, kSingly>(cx, g, A, lds_u32_2b_addr(cx.r0 + 192u + 4u * g), lds_u32_2b_addr(cx.r1 + 192u + 4u * g), S);
+        ib_groups16_step<NT>(cx, g, A, lds_u32_2b_addr(cx.r0 + 192u + 4u * g), lds_u32_2b_addr(cx.r1 + 192u + 4u * g), S);
       }
     }
     const float d0 = 0.25f * h2f_bits(lds_u16_addr(cx.r0 + 208u)), d1 = 0.25f * h2f_bits(lds_u16_addr(cx.r1 + 208u));
-    ib_groups16_finish<NT, kSingly>(cx, S, d0, d1, facc);
+    ib_groups16_finish<NT>(cx, S, d0, d1, facc);
   }
 };
 
@@ -345,7 +345,7 @@ struct IbQ3K {
 #pragma unroll
     for (int i = 0; i < 4; ++i) sc[i] = ((sc[i] | 0x80808080u) - 0x20202020u) ^ 0x80808080u;
   }
-  template <int NT, bool kSingly, int MT>
+  template <int NT, int MT>
   __device__ __forceinline__ static void block(const IbCtx& cx, float (&facc)[MT][4]) {
     uint32_t sc0[4], sc1[4], hm[2][2];  // hm: [s][row]
     scales(cx.r0, sc0);
@@ -375,11 +375,11 @@ struct IbQ3K {
               const int j = 2 * u + jj;
               A[2 * jj + s][r] = (((q[s][r] >> (2 * j)) & 0x03030303u) << 5) ^ ((((hm[s][r] >> (4 * c + j)) & 0x01010101u) << 7) ^ 0x80808080u);
             }
-        ib_groups16_step<NT, kSingly>(cx, 2 * c + u, A, sc0[2 * c + u], sc1[2 * c + u], S);
+        ib_groups16_step<NT>(cx, 2 * c + u, A, sc0[2 * c + u], sc1[2 * c + u], S);
       }
     }
     const float d0 = 0.03125f * h2f_bits(lds_u16_addr(cx.r0 + 108u)), d1 = 0.03125f * h2f_bits(lds_u16_addr(cx.r1 + 108u));
-    ib_groups16_finish<NT, kSingly>(cx, S, d0, d1, facc);
+    ib_groups16_finish<NT>(cx, S, d0, d1, facc);
   }
 };
 
@@ -389,7 +389,7 @@ struct IbQ2K {
   static constexpr bool kAligned = false;
   static constexpr IbAct kAct = kIbQ8K;
   static constexpr bool kSums = true;
-  template <int NT, bool kSingly, int MT>
+  template <int NT, int MT>
   __device__ __forceinline__ static void block(const IbCtx& cx, float (&facc)[MT][4]) {
     uint32_t am[4], sw[2][4];
 #pragma unroll
@@ -475,7 +475,7 @@ struct Ib32 {
       }
     }
   }
-  template <int NT, bool kSingly, int MT>
+  template <int NT, int MT>
   __device__ __forceinline__ static void block(const IbCtx& cx, float (&facc)[MT][4]) {
 #pragma unroll
     for (int g = 0; g < 4; ++g) {  // two 32-element blocks at a time
@@ -529,7 +529,7 @@ __device__ __forceinline__ void ib_block(const IbCtx& cx, float (&facc)[MT][4]) 
       return;
     }
   }
-  F::template block<NT, false>(cx, facc);
+  F::template block<NT>(cx, facc);
 }
 
 // kGrouped: the rows of many matrices' groups; else one matrix
@@ -818,8 +818,7 @@ __global__ void __launch_bounds__(32 * (MT > 4 ? kIbMaxWarps / 2 : kIbMaxWarps),
             cx.r1 = st + (uint32_t)((cx.gid + 8) * F::kPitch) + k1;
             cx.lm = st + (uint32_t)(((lane & 7) + (lane & 8)) * F::kPitch) + 16u * (lane >> 4);
             cx.act = abase + (uint32_t)((kpart * bpc + j) * slot_bytes);
-            if constexpr (kGrouped && MT > 4) F::template block<MT, true>(cx, facc);
-            else ib_block<F, kGrouped ? 1 : MT>(cx, facc);
+            ib_block<F, kGrouped ? 1 : MT>(cx, facc);
             __syncwarp();  // every lane has read the stage before any lane refills it
           }
           if (more) {

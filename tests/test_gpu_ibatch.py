@@ -39,7 +39,7 @@ def test_batch_edges_match_the_oracle(oracle, name):
 @pytest.mark.parametrize("counts,n,k", [
     ([0, 3, 0, 0, 1, 0, 0, 9] + [0] * 56, 293, 768),          # few groups: blocks of their own
     ([1] * 70 + [0] * 5 + [40] + [2] * 52, 37, 512),          # many: blocks that span several, one group in several passes
-    ([17, 0, 33, 24, 8, 130, 1, 16] * 5, 165, 2304),          # up to 64 rows a pass, and more
+    ([17, 0, 33, 24, 8, 130, 1, 16] * 5, 165, 2304),          # several passes of 32 rows
     ([26, 31, 12, 0, 25, 18, 32, 20] * 16, 85, 2048),         # some twenty rows each: sixteen warps a block
     ([0, 0, 1, 0], 37, 1280),                                 # a single row: planes, the sums converted as they are staged
 ])
