@@ -640,6 +640,7 @@ int32_t ibatch_fmt(int type, int n_groups, int64_t n, int64_t k, const void* w, 
   int mt = p.rows_cap / 8;
   if (mt > 4) mt = mt <= 6 ? 6 : 8;
   if (kGrouped && mt == 3) mt = 4;
+  if (!act.rec && mt > 1) return kNotSupported;  // can't be: planes are a single row's
   const cudaError_t e = ibatch_launch(type, mt, kGrouped, p, (unsigned)blocks, warps, smem, di->max_smem_optin, stream);
   return e == cudaSuccess ? kOk : kLaunchFailure;
 }

@@ -165,7 +165,7 @@ struct IbCtx {
 };
 
 // The activation tiles of a step, in parts that run together: with a branch around each tile, none of one tile's loads and
-// products can be issued under the latency of another's (Q4_K 11008 x 4096, 48 rows: 45 us, with parts 36); with all of eight,
+// products can be issued under the latency of another's (Q4_K 11008 x 4096, 48 rows: 45 us, with parts 35); with all of eight,
 // or three of the sixteen-group formats at the sixteen-warp form's 128 registers, the registers spill (64 rows: 51 and 77 us).
 __host__ __device__ constexpr int ib_part(int nt, int small, int large) {
   return nt <= 2 ? nt : nt <= 4 ? (small < nt ? small : nt) : nt <= 6 ? nt : large;
@@ -204,18 +204,14 @@ struct IbQ45K {
   static constexpr bool kSums = true;  // reads the 16-element sums
   template <int NT, int MT>
   __device__ __forceinline__ static void block(const IbCtx& cx, float (&facc)[MT][4]) {
-    const uint4 h0 = lds128(cx.r0), h1 = lds128(cx.r1);
-    // eight 6-bit scales / mins per row as bytes of two words (get_scale_min_k4, fuel-quantized/src/utils.rs:50-60)
-    const uint32_t sc0[2] = {h0.y & 0x3f3f3f3fu, (h0.w & 0x0f0f0f0fu) | (((h0.y >> 6) & 0x03030303u) << 4)};
-    const uint32_t mn0[2] = {h0.z & 0x3f3f3f3fu, ((h0.w >> 4) & 0x0f0f0f0fu) | (((h0.z >> 6) & 0x03030303u) << 4)};
-    const uint32_t sc1[2] = {h1.y & 0x3f3f3f3fu, (h1.w & 0x0f0f0f0fu) | (((h1.y >> 6) & 0x03030303u) << 4)};
-    const uint32_t mn1[2] = {h1.z & 0x3f3f3f3fu, ((h1.w >> 4) & 0x0f0f0f0fu) | (((h1.z >> 6) & 0x03030303u) << 4)};
-    const float d0 = h2f_bits(h0.x & 0xffffu), dm0 = h2f_bits(h0.x >> 16);
-    const float d1 = h2f_bits(h1.x & 0xffffu), dm1 = h2f_bits(h1.x >> 16);
-    uint32_t am[4];  // minimum of 16-element group i = minimum of sub-block i / 2: this lane's groups 2 tig, + 1, + 8, + 9
+    // Eight 6-bit scales per row as bytes of two words (get_scale_min_k4, fuel-quantized/src/utils.rs:50-60). The rest of the
+    // block's first 16 bytes is read again behind the loop: held across it, it takes registers that the two-tile form spills
+    // (4096 x 11008, 16 rows: 20.6 us, read again 19.9).
+    uint32_t sc0[2], sc1[2];
     {
-      const int a = ib_byte(mn0[0], cx.tig), b = ib_byte(mn1[0], cx.tig), c = ib_byte(mn0[1], cx.tig), e = ib_byte(mn1[1], cx.tig);
-      am[0] = ib_h2(a, a), am[1] = ib_h2(b, b), am[2] = ib_h2(c, c), am[3] = ib_h2(e, e);
+      const uint4 h0 = lds128(cx.r0), h1 = lds128(cx.r1);
+      sc0[0] = h0.y & 0x3f3f3f3fu, sc0[1] = (h0.w & 0x0f0f0f0fu) | (((h0.y >> 6) & 0x03030303u) << 4);
+      sc1[0] = h1.y & 0x3f3f3f3fu, sc1[1] = (h1.w & 0x0f0f0f0fu) | (((h1.y >> 6) & 0x03030303u) << 4);
     }
     uint32_t hq[4];
     if constexpr (kFive) ldmatrix_x4(hq, cx.lm + 16u);
@@ -241,7 +237,13 @@ struct IbQ45K {
         mma_u8_k32<true>(cl, lo, b[0], b[1]);
         mma_u8_k32<true>(ch, hi, b[2], b[3]);
         int (&T)[4] = S[mt];
-        if (g == 0) {
+        // one product at a time where many tiles run together: fewer registers (48 rows: 33.0 -> 32.5 us, 32 rows 28.8 -> 27.7;
+        // the two-tile form 19.9 -> 21.2)
+        if constexpr (NT > 2) {
+          if (g == 0) T[0] = cl[0] * s0l, T[1] = cl[1] * s0l, T[2] = cl[2] * s1l, T[3] = cl[3] * s1l;
+          else T[0] += cl[0] * s0l, T[1] += cl[1] * s0l, T[2] += cl[2] * s1l, T[3] += cl[3] * s1l;
+          T[0] += ch[0] * s0h, T[1] += ch[1] * s0h, T[2] += ch[2] * s1h, T[3] += ch[3] * s1h;
+        } else if (g == 0) {
           T[0] = cl[0] * s0l + ch[0] * s0h, T[1] = cl[1] * s0l + ch[1] * s0h;
           T[2] = cl[2] * s1l + ch[2] * s1h, T[3] = cl[3] * s1l + ch[3] * s1h;
         } else {
@@ -249,6 +251,16 @@ struct IbQ45K {
           T[2] += cl[2] * s1l + ch[2] * s1h, T[3] += cl[3] * s1l + ch[3] * s1h;
         }
       }
+    }
+    const uint4 h0 = lds128(cx.r0), h1 = lds128(cx.r1);
+    const uint32_t mn0[2] = {h0.z & 0x3f3f3f3fu, ((h0.w >> 4) & 0x0f0f0f0fu) | (((h0.z >> 6) & 0x03030303u) << 4)};
+    const uint32_t mn1[2] = {h1.z & 0x3f3f3f3fu, ((h1.w >> 4) & 0x0f0f0f0fu) | (((h1.z >> 6) & 0x03030303u) << 4)};
+    const float d0 = h2f_bits(h0.x & 0xffffu), dm0 = h2f_bits(h0.x >> 16);
+    const float d1 = h2f_bits(h1.x & 0xffffu), dm1 = h2f_bits(h1.x >> 16);
+    uint32_t am[4];  // minimum of 16-element group i = minimum of sub-block i / 2: this lane's groups 2 tig, + 1, + 8, + 9
+    {
+      const int a = ib_byte(mn0[0], cx.tig), b = ib_byte(mn1[0], cx.tig), c = ib_byte(mn0[1], cx.tig), e = ib_byte(mn1[1], cx.tig);
+      am[0] = ib_h2(a, a), am[1] = ib_h2(b, b), am[2] = ib_h2(c, c), am[3] = ib_h2(e, e);
     }
     FQ_IB_TILES(4, 4)
       ib_finish_min(cx, mt, am, S[mt], d0, dm0, d1, dm1, facc);
@@ -270,11 +282,13 @@ __device__ __forceinline__ void ib_groups16_step(const IbCtx& cx, int g, const u
     ib_b64(cx, mt, g, b);
     int (&T)[4] = S[mt];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      int c[4];
+    for (int i = 0; i < 4; i += 2) {
+      int c[4], e[4];
       mma_s8_k16(c, A[i][0], A[i][1], b[i]);
+      mma_s8_k16(e, A[i + 1][0], A[i + 1][1], b[i + 1]);
       if (g == 0 && i == 0) T[0] = c[0] * s0[i], T[1] = c[1] * s0[i], T[2] = c[2] * s1[i], T[3] = c[3] * s1[i];
       else T[0] += c[0] * s0[i], T[1] += c[1] * s0[i], T[2] += c[2] * s1[i], T[3] += c[3] * s1[i];
+      T[0] += e[0] * s0[i + 1], T[1] += e[1] * s0[i + 1], T[2] += e[2] * s1[i + 1], T[3] += e[3] * s1[i + 1];
     }
   }
 }
@@ -710,6 +724,9 @@ __global__ void __launch_bounds__(32 * (MT > 4 ? kIbMaxWarps / 2 : kIbMaxWarps),
   // the chunk of share s / bpc: the rows' records, one bulk copy (a lane of warp 0 each). Rows past `ac` keep whatever is
   // there: a row is a column of the MMAs' results, and theirs are not stored.
   constexpr int kRec = ib_rec(F::kAct);
+  // Planes: a single row, so the forms for more tiles have no code for them. (Nor could the two-tile form, but its registers
+  // came out worse without: Q4_K 4096 x 11008 at 16 rows 19.9 -> 20.3 us.)
+  auto records = [&]() -> bool { return MT > 2 || p.act.rec; };
   int slot_bytes, bpc, n_chunks;
   auto stage_acts = [&](int a0, int ac, int c, int buf) {
     const uint32_t base = (uint32_t)(p.act_off + buf * p.act_buf);
@@ -718,7 +735,7 @@ __global__ void __launch_bounds__(32 * (MT > 4 ? kIbMaxWarps / 2 : kIbMaxWarps),
       const int sh = s / bpc, b0 = sh * p.share_q + (sh < p.share_rem ? sh : p.share_rem), j = c * bpc + s - sh * bpc;
       return j < p.share_q + (sh < p.share_rem) ? b0 + j : -1;
     };
-    if (p.act.rec) {
+    if (records()) {
       if (warp == 0) {
         int mine = 0;
         for (int s = lane; s < slots; s += 32) mine += slot_block(s) >= 0;
@@ -752,7 +769,7 @@ __global__ void __launch_bounds__(32 * (MT > 4 ? kIbMaxWarps / 2 : kIbMaxWarps),
   };
   uint32_t phases = 0;  // bit b: parity of buffer b's next fill
   auto acts_landed = [&](int buf) {
-    if (p.act.rec) {
+    if (records()) {
       if (!mbar_wait_bounded(&full[buf], (phases >> buf) & 1u)) record_dev_error(kErrFullWait);  // carries on: the host sees the code
       phases ^= 1u << buf;
     }
@@ -779,7 +796,7 @@ __global__ void __launch_bounds__(32 * (MT > 4 ? kIbMaxWarps / 2 : kIbMaxWarps),
       cx.nt = (ac + 7) >> 3;
       if (pass > 0 || !first) __syncthreads();  // the previous pass's activations are done with
       stage_acts(a0, ac, 0, 0);
-      if (!p.act.rec) {
+      if (!records()) {
         ib_wait(0);
         __syncthreads();
       }
@@ -822,7 +839,7 @@ __global__ void __launch_bounds__(32 * (MT > 4 ? kIbMaxWarps / 2 : kIbMaxWarps),
             __syncwarp();  // every lane has read the stage before any lane refills it
           }
           if (more) {
-            if (!p.act.rec) ib_wait(0);
+            if (!records()) ib_wait(0);
             __syncthreads();
             buf ^= 1;
             acts_landed(buf);
