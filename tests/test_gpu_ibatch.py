@@ -69,3 +69,25 @@ def test_groups_match_the_oracle(oracle, name, counts, n, k):
             r = slice(off[i], off[i] + c)
             assert_matmul_close(got[r], oracle.matmul(ot, x[r], wb.reshape(-1)[i * per:(i + 1) * per], n), (name, i, c))
     assert ops.device_error() == 0
+
+
+@pytest.mark.parametrize("name", FORMATS)
+def test_a_row_that_is_not_finite_stays_by_itself(name):
+    """Rows are columns of the MMAs: infinities and NaN in some rows change no bit of the others, in the same call or the next."""
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from fuel_b200 import GgmlDType as T, ops
+    t, n, k = getattr(T, name), 83, 1536
+    gen = torch.Generator(device="cuda").manual_seed(17)
+    w = ops.quantize_weights(t, torch.randn(n, k, generator=gen, device="cuda"))
+    for m in (2, 7, 16):
+        x = torch.randn(m, k, generator=gen, device="cuda")
+        want = ops.qmatmul(t, w, n, x)
+        bad = x.clone()
+        bad[m // 2, 3], bad[m // 2, 700] = float("inf"), float("nan")
+        got = ops.qmatmul(t, w, n, bad)
+        rest = [i for i in range(m) if i != m // 2]
+        assert torch.equal(got[rest], want[rest]), m
+        ops.qmatmul(t, w, n, torch.full((16, k), float("nan"), device="cuda"))
+        assert torch.equal(ops.qmatmul(t, w, n, x), want), m
+    assert ops.device_error() == 0
