@@ -1724,8 +1724,10 @@ int32_t fuelq_moe_combine(const float* y_pairs, const int32_t* topk_ids, const f
     return kInvalidProblem;
   if (n_tokens == 0) return kOk;
   if (!y_pairs || !topk_ids || !topk_weights || !out) return kInvalidProblem;
-  // a few tokens: their columns over several thread blocks
-  const unsigned parts = n_tokens >= 148 ? 1 : (unsigned)((n + 1023) / 1024 < 16 ? (n + 1023) / 1024 : 16);
+  DeviceInfo* di;
+  if (!device_info(&di)) return kLaunchFailure;
+  // fewer tokens than SMs: their columns over several thread blocks
+  const unsigned parts = n_tokens >= di->sm_count ? 1 : (unsigned)((n + 1023) / 1024 < 16 ? (n + 1023) / 1024 : 16);
   const cudaError_t e = launch(moe_combine_kernel, dim3((unsigned)n_tokens, parts), dim3(256), 0, (cudaStream_t)stream, y_pairs,
                                (const int*)topk_ids, topk_weights, (int)top_k, (int)n, out);
   return e == cudaSuccess ? kOk : kLaunchFailure;
