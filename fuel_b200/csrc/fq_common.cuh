@@ -265,8 +265,7 @@ __device__ __forceinline__ uint32_t lds_u16(const uint8_t* p) {
 }
 __device__ __forceinline__ float h2f_bits(uint32_t h) { return __half2float(__ushort_as_half((unsigned short)h)); }
 
-// defined once: the library is a single translation unit
-static __device__ int g_fq_dev_error = 0;  // one in each of the library's translation units
+static __device__ int g_fq_dev_error = 0;  // one in each of the library's translation units; the host reads them all
 __device__ __forceinline__ void record_dev_error(int code) { atomicCAS(&g_fq_dev_error, 0, code); }
 
 #endif  // __CUDACC__

@@ -1,5 +1,5 @@
 // libfuelq.so — C ABI over the sm_100a kernels (see include/fuelq.h for the contract).
-// Single translation unit: the kernels live in the .cuh files included below.
+// The kernels live in the .cuh files included below; those of ibatch.cuh are compiled beside this file, in ibatch.cu.
 #include "../../include/fuelq.h"
 
 #include <cuda_bf16.h>
@@ -645,7 +645,8 @@ int32_t ibatch_fmt(int type, int n_groups, int64_t n, int64_t k, const void* w, 
   return e == cudaSuccess ? kOk : kLaunchFailure;
 }
 
-// kNotSupported when the shape has no plan here (the caller falls back)
+// kNotSupported when the shape has no plan here: the grouped form falls back to the dp4a kernel; for rows kept as records every
+// plan fits (one share of k, one block a chunk, two stages: 161 KB)
 int32_t ibatch_impl(int type, int n_groups, int64_t n, int64_t k, const void* w, const ActPlanes& act, const int* offsets,
                     int64_t n_rows, const int* out_rows, float* y, cudaStream_t stream, bool early_w) {
   if (k % 256 || n > INT32_MAX - 64 || n_groups > 65535 || n_rows > (1 << 28)) return kNotSupported;

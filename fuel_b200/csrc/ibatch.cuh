@@ -724,8 +724,8 @@ __global__ void __launch_bounds__(32 * (MT > 4 ? kIbMaxWarps / 2 : kIbMaxWarps),
   // the chunk of share s / bpc: the rows' records, one bulk copy (a lane of warp 0 each). Rows past `ac` keep whatever is
   // there: a row is a column of the MMAs' results, and theirs are not stored.
   constexpr int kRec = ib_rec(F::kAct);
-  // Planes: a single row, so the forms for more tiles have no code for them. (Nor could the two-tile form, but its registers
-  // came out worse without: Q4_K 4096 x 11008 at 16 rows 19.9 -> 20.3 us.)
+  // Planes hold a single row, so the forms for many tiles have no code for them. The two-tile form needs none either, but its
+  // registers came out worse without: Q4_K 4096 x 11008 at 16 rows 19.9 -> 20.3 us.
   auto records = [&]() -> bool { return MT > 2 || p.act.rec; };
   int slot_bytes, bpc, n_chunks;
   auto stage_acts = [&](int a0, int ac, int c, int buf) {

@@ -4,6 +4,12 @@
  * Status codes as in fuelq.h; fuelq_last_error() returns the message of the calling thread's
  * last failure. Unlike the kernel-level entry points in fuelq.h these own device memory
  * (the weight blocks and a reusable activation workspace), like the reference's storage types.
+ *
+ * The workspace of fuelq_qmatmul_forward: the weights made on one stream share it (at least 1 MiB; it grows at least twofold
+ * and keeps the smaller buffers, below four times the largest need in all) until the last of them is freed. A weight has
+ * workspace of its own for calls recorded into a CUDA graph, which may be replayed beside other calls, and for calls made
+ * with cudaStreamPerThread from another thread than the one that made it. Graphs that hold a weight's calls must not be
+ * replayed at the same time as one another, nor after the weight is freed. Freed memory goes back to the driver at once.
  */
 #ifndef FUELQ_HOST_H_
 #define FUELQ_HOST_H_
