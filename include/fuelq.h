@@ -61,8 +61,8 @@ int32_t fuelq_block_bytes(int32_t ggml_type);
                                     predecessor's tail (default 0: only the later kernels of a call do) */
 #define FUELQ_OPT_DECODE_MAX_M 2 /* largest m_total routed to the integer kernels; above it the tensor-core GEMM runs
                                     (every block format, k a multiple of 64). 0 (default) = the library's choice: 16,
-                                    and 64 for Q4_K / Q5_K / Q6_K / Q8_0 with k a multiple of 256 (the integer tensor-core
-                                    kernel is still the faster of the two there).
+                                    and 64 for Q4_K / Q5_K / Q6_K / Q8_0 with k a multiple of 256 (one pass of the integer
+                                    tensor-core kernel over the weights, the faster of the two up to there).
                                     Any positive value is taken as given */
 #define FUELQ_OPT_DECODE_GRID 3  /* CTAs for the decode kernel; 0 = two per SM (default) */
 #define FUELQ_OPT_DECODE_KERNEL 4 /* 0 = pick per problem (default); 1 = generic decode kernel (activations read
